@@ -89,7 +89,7 @@ struct SceneHost {
   SceneDev d{};  // device pointers filled after allocation
   // arena offsets
   size_t o_sf, o_su, o_pos, o_rot, o_ppos, o_prot, o_lv, o_av, o_spos, o_srot, o_alo, o_ahi, o_art, o_cnt, o_stats,
-      o_params, o_craw, o_con, o_ckeys, o_rows, o_slots, o_warm, o_sched, o_tw, o_imp, o_aqd, o_tscr;
+      o_params, o_craw, o_con, o_ckeys, o_rows, o_slots, o_pk, o_plam, o_warm, o_sched, o_tw, o_imp, o_aqd, o_tscr;
   // Device-wide radix sort of a scene whose padded keys may exceed the block sort's shared array.
   bool large_sort = false;
   uint32_t sort_tiles = 0;
@@ -302,6 +302,7 @@ int build_scene(SceneHost& s, const steel_scene_desc& in, Layout& L, uint32_t th
     s.o_rctr = L.take(4ull * RS_DIGITS);
   }
   s.o_rows = L.take((size_t)MAXC * d.ROWS * 16); s.o_slots = L.take((size_t)MAXC * 2 * 16);
+  s.o_pk = L.take(((size_t)MAXC / 8u + d.NCOL + 8u) * PK_TILE); s.o_plam = L.take((size_t)MAXC * 4);
   s.o_warm = L.take(s.warm_words * 4);
   s.o_sched = L.take(s.sched_words * 4);
   s.o_tw = L.take((size_t)NB * 32); s.o_imp = L.take((size_t)NB * 32);
@@ -391,7 +392,8 @@ void drop_graph(steel_batch* b) {
 // Shared-memory staging flags of a scene under a per-block budget of dynamic shared memory (0: the
 // per-part caps alone). Link blocks first, then twists and impulses, qd, and the color masks; a part
 // is staged when it is under its cap and both kernels' layouts stay within the budget.
-uint32_t stage_flags(const SceneDev& d, uint32_t budget) {
+// body_cap: the cap on twists and impulses.
+uint32_t stage_flags(const SceneDev& d, uint32_t budget, uint64_t body_cap) {
   const uint64_t lim = budget ? budget : ~0ull;
   auto fits = [&](uint32_t f) {
     return prep_smem_layout(f, d.NL, d.NB, d.NCOLW, d.NCOL).total <= lim &&
@@ -399,7 +401,7 @@ uint32_t stage_flags(const SceneDev& d, uint32_t budget) {
   };
   uint32_t st = 0u;
   if (d.NL > 0u && 4ull * d.NL * 268u <= STAGE_LINK_CAP && fits(st | STAGE_LINKS)) st |= STAGE_LINKS;
-  if (64ull * d.NB <= STAGE_BODY_CAP && fits(st | STAGE_BODIES)) st |= STAGE_BODIES;
+  if (64ull * d.NB <= body_cap && fits(st | STAGE_BODIES)) st |= STAGE_BODIES;
   if (4ull * d.ND <= STAGE_QD_CAP && fits(st | STAGE_QD)) st |= STAGE_QD;
   if (4ull * d.NB * d.NCOLW <= STAGE_WMASK_CAP && fits(st | STAGE_WMASK)) st |= STAGE_WMASK;
   return st;
@@ -421,7 +423,7 @@ int team_blocks_for(const steel_batch* b, uint32_t req, bool strict, uint32_t* o
       return fail(STEEL_E_INVALID, "team launches use 512-thread blocks; the batch's tiles have " + std::to_string(T));
     return STEEL_OK;
   }
-  const int per_sm = std::min(solve_team_blocks_per_sm(T, b->bd.solve_smem),
+  const int per_sm = std::min(solve_team_blocks_per_sm(T, b->bd.team_smem),
                               prepare_team_blocks_per_sm(T, b->bd.prep_smem));
   const uint32_t cap = per_sm > 0 ? (uint32_t)per_sm * (uint32_t)b->ctx->sms : 0u;
   uint32_t n = 0u;
@@ -583,13 +585,26 @@ int apply_tiles(steel_batch* b, const steel_tiles& t) {
   if (t.stream_groups > 8u) return fail(STEEL_E_INVALID, "at most 8 stream groups");
   const uint32_t n = (uint32_t)b->sc.size();
   std::vector<uint32_t> stages(n);
-  size_t prep = 0, solve = 0;
+  size_t prep = 0, solve = 0, team = 0;
+  // Dynamic shared memory a solve block may use without lowering the blocks per SM that this batch
+  // can keep resident (a batch of no more scenes than SMs: one block with all of it). What the
+  // scene's staging leaves holds its packed rows, so the solve reads them at shared-memory latency.
+  const uint32_t resident = std::min<uint32_t>(blocks_per_sm_of(t.block_threads),
+                                               (n + (uint32_t)b->ctx->sms - 1u) / (uint32_t)b->ctx->sms);
+  const size_t room = std::min<size_t>(t.smem_budget ? t.smem_budget : SMEM_PER_SM, solve_smem_room(resident));
+  const uint64_t body_cap = std::max<uint64_t>(STAGE_BODY_CAP, room / 3u);
   for (uint32_t i = 0; i < n; i++) {
     SceneDev& d = b->sc[i].d;
-    d.stage = stage_flags(d, t.smem_budget);
+    d.stage = stage_flags(d, t.smem_budget, body_cap);
     stages[i] = d.stage;
     prep = std::max<size_t>(prep, prep_smem_layout(d.stage, d.NL, d.NB, d.NCOLW, d.NCOL).total);
-    solve = std::max<size_t>(solve, solve_smem_layout(d.stage, d.NB, d.ND, d.NCOL, d.NL).total);
+    team = std::max<size_t>(team, solve_smem_layout(0u, d.NB, d.ND, d.NCOL, d.NL).total);
+    const size_t staged = solve_smem_layout(d.stage, d.NB, d.ND, d.NCOL, d.NL).total;
+    // Room for 8 rows per free body and 2 per link, a partly filled tile per color; more L1 is left
+    // to the articulated passes that way than by reserving the capacity MAXC.
+    const uint32_t free_bodies = d.NB - std::min(d.NB, d.NL);
+    const size_t tiles = free_bodies + d.NL / 4u + std::min(d.NCOL, free_bodies) + 2u;
+    solve = std::max(solve, std::max(staged, std::min(room, staged + 128u + tiles * PK_TILE)));
   }
   CU(cudaSetDevice(b->ctx->device));
   cudaStream_t st = b->ctx->stream;
@@ -602,6 +617,7 @@ int apply_tiles(steel_batch* b, const steel_tiles& t) {
   CU(cudaStreamSynchronize(st));
   b->bd.prep_smem = (uint32_t)prep;
   b->bd.solve_smem = (uint32_t)solve;
+  b->bd.team_smem = (uint32_t)team;
   b->bd.block_threads = t.block_threads;
   b->narrow_blocks = (uint32_t)b->ctx->sms * (t.narrow_blocks_per_sm ? t.narrow_blocks_per_sm : narrow_max);
   const uint32_t want_groups = t.stream_groups > 1u ? t.stream_groups : 1u;
@@ -728,6 +744,7 @@ int steel_batch_create(steel_ctx* ctx, const steel_scene_desc* scenes, uint32_t 
     d.params = at<Params>(A, s.o_params);
     d.craw = at<float4>(A, s.o_craw); d.con = at<float4>(A, s.o_con); d.ckeys = at<uint4>(A, s.o_ckeys);
     d.rows = at<float4>(A, s.o_rows); d.slots = at<float4>(A, s.o_slots);
+    d.pk = at<char>(A, s.o_pk); d.plam = at<float>(A, s.o_plam);
     d.warm_tab = at<uint32_t>(A, s.o_warm); d.sched = at<uint32_t>(A, s.o_sched);
     d.tw = at<float4>(A, s.o_tw); d.imp = at<float4>(A, s.o_imp); d.aqd = at<float>(A, s.o_aqd);
     d.tscr = at<float>(A, s.o_tscr);
@@ -753,6 +770,7 @@ int steel_batch_create(steel_ctx* ctx, const steel_scene_desc* scenes, uint32_t 
   BatchDev& bd = b->bd;
   bd.scenes = at<SceneDev>(A, b->o_scenes);
   bd.nscenes = n;
+  bd.sms = (uint32_t)ctx->sms;
   bd.nshapes = (uint32_t)b->shape_scene.size();
   bd.shape_scene = at<uint32_t>(A, b->o_shape_scene);
   bd.shape_local = at<uint32_t>(A, b->o_shape_local);

@@ -26,6 +26,8 @@ struct BatchDev {
   uint32_t* error;            // [1] first device-side error code (0 = none)
   uint32_t prep_smem;         // dynamic shared memory of k_prepare / k_solve launches (bytes)
   uint32_t solve_smem;
+  uint32_t sms;               // SMs of the device
+  uint32_t team_smem;         // dynamic shared memory of k_solve_team launches (nothing staged)
   uint32_t art_f64;           // some scene has ART_F64: launch the prepare instances that carry it
   uint32_t solve_ext;         // some scene has ANG_ART or CTI: launch the solve instances that carry them
   uint32_t block_threads;     // threads per prepare / solve block (one of BLOCK_SIZES)
@@ -93,6 +95,7 @@ constexpr uint32_t TEAM_WAIT_LIMIT = 1u << 22;  // polls of a team launch's grid
 // TEAM_MIN_BODIES bodies or TEAM_MIN_ARTS articulations; such a scene's per-thread scratch has
 // slices for TEAM_SCRATCH_BLOCKS blocks, so the prepare's scratch passes spread over that many.
 constexpr uint32_t TEAM_MIN_BODIES = 2048u, TEAM_MIN_ARTS = 64u, TEAM_SCRATCH_BLOCKS = 32u;
+constexpr uint32_t PK_TILE = 15u * 128u;  // bytes of a tile of 8 packed solver rows: 15 float4 fields (solve.cuh)
 struct RadixDev {
   uint4* keys[2];     // ping-pong key buffers [MAXC] (x pair, y feature, z hash, w raw index)
   uint32_t* status;   // [RS_DIGITS][tiles][256] look-back words: bits 30-31 flag (1 tile count, 2 prefix)
@@ -110,6 +113,18 @@ constexpr uint32_t STAGE_LINK_CAP = 44u * 1024u;   // link blocks (NL * 1072 B)
 constexpr uint32_t STAGE_BODY_CAP = 8u * 1024u;    // twists + impulses (NB * 64 B)
 constexpr uint32_t STAGE_QD_CAP = 8u * 1024u;      // generalized velocities of the solve (ND * 4 B)
 constexpr uint32_t STAGE_WMASK_CAP = 16u * 1024u;  // per-body color masks (NB * NCOLW words)
+// Shared memory of an SM, and the dynamic part of each of `resident` solve blocks: a block takes 1 KB
+// of system use and the kernel's static arrays (under 5 KB) besides, and 227 KB at most.
+constexpr size_t SMEM_PER_SM = 228u * 1024u;
+constexpr size_t solve_smem_room(uint32_t resident) {
+  return (SMEM_PER_SM / (resident > 0u ? resident : 1u) - 6u * 1024u) & ~(size_t)127u;
+}
+// Percent of an SM's shared memory that a solve launch's resident blocks use.
+inline unsigned int solve_carveout(const BatchDev& b) {
+  const uint32_t per_sm = blocks_per_sm_of(b.block_threads), need = (b.nlaunch + b.sms - 1u) / b.sms;
+  const size_t bytes = (size_t)(need < per_sm ? need : per_sm) * (b.solve_smem + 6u * 1024u);
+  return bytes >= SMEM_PER_SM ? 100u : (unsigned int)((100u * bytes + SMEM_PER_SM - 1u) / SMEM_PER_SM);
+}
 // Byte offsets of a scene's parts in k_prepare's dynamic shared memory: link blocks (if staged),
 // color counts, color masks (if staged).
 struct PrepSmem { uint32_t links, wcount, wmask, total; };

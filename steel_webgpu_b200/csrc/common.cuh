@@ -221,6 +221,8 @@ struct SceneDev {
   uint4* ckeys;                      // sort scratch [MAXC]
   float4* rows;                      // row records [MAXC * ROWS]
   float4* slots;                     // slot table [MAXC * 2]
+  char* pk;                          // solve: rows packed by color in tiles of 8 (solve.cuh)
+  float* plam;                       // solve: normal impulses in row order, 0 for rows outside a patch [MAXC]
   uint32_t* warm_tab;                // warm table: 10*WH + 30*AH words
   uint32_t* sched;                   // scheduling arrays, offsets below
   uint32_t S_UNITOF, S_DSLOT, S_CORDER, S_UKEY, S_USTART0, S_USIZE, S_USTART, S_RK0, S_RK1, S_RK2, S_BPC, S_LEAD,

@@ -57,7 +57,7 @@ void launch_solve_t<STEEL_BLOCK>(const BatchDev& b, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(b.team_blocks);
     cfg.blockDim = dim3(STEEL_BLOCK);
-    cfg.dynamicSmemBytes = b.solve_smem;
+    cfg.dynamicSmemBytes = b.team_smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;  // every block resident: the grid barrier's guarantee
@@ -70,8 +70,21 @@ void launch_solve_t<STEEL_BLOCK>(const BatchDev& b, cudaStream_t st) {
     return;
   }
 #endif
-  if (b.solve_ext) STEEL_NS::k_solve<true><<<b.nlaunch, STEEL_BLOCK, b.solve_smem, st>>>(b);
-  else STEEL_NS::k_solve<false><<<b.nlaunch, STEEL_BLOCK, b.solve_smem, st>>>(b);
+  // The launch asks for the shared memory its resident blocks use and leaves the rest to L1, which
+  // the articulated passes read through (without the hint the driver provides for as many blocks as
+  // the registers allow).
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(b.nlaunch);
+  cfg.blockDim = dim3(STEEL_BLOCK);
+  cfg.dynamicSmemBytes = b.solve_smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  at[0].val.sharedMemCarveout = solve_carveout(b);
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (b.solve_ext) cudaLaunchKernelEx(&cfg, STEEL_NS::k_solve<true>, b);
+  else cudaLaunchKernelEx(&cfg, STEEL_NS::k_solve<false>, b);
 }
 template <>
 int solve_team_blocks_per_sm_t<STEEL_BLOCK>(size_t smem_bytes) {

@@ -182,18 +182,32 @@ struct SolverT {
     const f2 tf = clip_cone(lt + tangent_step(ut0 + gnt * (ln - lam.x), g1), mu * ln);
     return mf3(ln, tf.x, tf.y);
   }
-  // Friction pair update on its 2x2 block with a disk bound (wgsl.js:2952-3011).
+  // Friction pair update on its 2x2 block with a disk bound (wgsl.js:2952-3011), in two parts: the
+  // block's scaled eigenvalues and first eigenvector, which depend on the row alone, and the
+  // update. A row's block does not change during a solve, so packed rows keep its FricEig.
+  struct FricEig { float scale, largest, smallest, vx, vy; };
+  static __device__ FricEig fric_eig(float a0, float c0, float d0) {
+    FricEig e;
+    e.scale = fmx(fmx(a0, d0), 1e-20f);
+    float a = a0 / e.scale, c = c0 / e.scale, d = d0 / e.scale;
+    e.largest = 0.5f * ((a + d) + sqrtf((a - d) * (a - d) + (4.0f * c) * c));
+    e.smallest = e.largest > 0.0f ? fmx((a * d - c * c) / e.largest, 0.0f) : 0.0f;
+    float vx = c, vy = e.largest - a;
+    if (a >= d) { vx = e.largest - d; vy = c; }
+    float vn = sqrtf(vx * vx + vy * vy);
+    if (vn > 0.0f) { vx /= vn; vy /= vn; } else { vx = 1.0f; vy = 0.0f; }
+    e.vx = vx;
+    e.vy = vy;
+    return e;
+  }
   static __device__ f2 friction_pair(float a0, float c0, float d0, float r0, float r1, float old0, float old1,
                                      float radius, float omega) {
     if (radius <= 0.0f) return mf2(0.0f, 0.0f);
-    float scale = fmx(fmx(a0, d0), 1e-20f);
-    float a = a0 / scale, c = c0 / scale, d = d0 / scale;
-    float largest = 0.5f * ((a + d) + sqrtf((a - d) * (a - d) + (4.0f * c) * c));
-    float smallest = largest > 0.0f ? fmx((a * d - c * c) / largest, 0.0f) : 0.0f;
-    float vx = c, vy = largest - a;
-    if (a >= d) { vx = largest - d; vy = c; }
-    float vn = sqrtf(vx * vx + vy * vy);
-    if (vn > 0.0f) { vx /= vn; vy /= vn; } else { vx = 1.0f; vy = 0.0f; }
+    return fric_solve(fric_eig(a0, c0, d0), r0, r1, old0, old1, radius, omega);
+  }
+  static __device__ f2 fric_solve(const FricEig& e, float r0, float r1, float old0, float old1, float radius,
+                                  float omega) {
+    const float scale = e.scale, largest = e.largest, smallest = e.smallest, vx = e.vx, vy = e.vy;
     float r0r = (vx * r0 + vy * r1) / scale;
     float r1r = ((-vy) * r0 + vx * r1) / scale;
     f2 res = mf2(old0, old1);
@@ -345,6 +359,35 @@ struct SolverT {
     rows[o + 21u] = make_float4(nl5[2], nl5[3], nl5[4], 0.0f);
     return AngOut{ta[0], ta[1], tb[0], tb[1], nl5[0], nl5[1]};
   }
+  // A free body's spin and rolling rows of contact row `row` under normal load nl2.
+  // Twists go in and out by value, so the caller's stay in registers.
+  struct Twists { f3 ta0, ta1, tb0, tb1; };
+  __device__ __noinline__ Twists free_angular(uint32_t row, int a, int b, f3 n, f3 t1, f3 t2, float nl2, f3 ta0, f3 ta1,
+                                              f3 tb0, f3 tb1) const {
+    f3 ta[2] = {ta0, ta1}, tb[2] = {tb0, tb1};
+    float4* R = S.rows + (size_t)row * S.ROWS;
+    const float4 g = R[19], la = R[21], ri = R[20];
+    const f3 wrel = tb[1] - ta[1];
+    const float ns = clmp(la.x - dot(n, wrel) * g.z, (-g.x) * nl2, g.x * nl2);
+    const float ds = ns - la.x;
+    ta[0] += v3(R[22]) * ds; ta[1] += v3(R[23]) * ds;
+    tb[0] += v3(R[24]) * ds; tb[1] += v3(R[25]) * ds;
+    const f3 w2 = tb[1] - ta[1];
+    const float u1 = dot(t1, w2), u2 = dot(t2, w2);
+    f2 lr = mf2(la.y, la.z) - mf2(ri.x * u1 + ri.y * u2, ri.y * u1 + ri.z * u2);
+    const float rl = g.y * nl2;
+    if (len(lr) > rl) lr = lr * (rl / fmx(len(lr), 1e-12f));
+    const float d1 = lr.x - la.y, d2 = lr.y - la.z;
+    ta[0] += v3(R[26]) * d1 + v3(R[30]) * d2;
+    ta[1] += v3(R[27]) * d1 + v3(R[31]) * d2;
+    tb[0] += v3(R[28]) * d1 + v3(R[32]) * d2;
+    tb[1] += v3(R[29]) * d1 + v3(R[33]) * d2;
+    R[21] = make_float4(ns, lr.x, lr.y, 0.0f);
+    const f3 tq = (n * ds + t1 * d1) + t2 * d2;
+    add_imp(a, sp3(0.0f), -tq);
+    add_imp(b, sp3(0.0f), tq);
+    return Twists{ta[0], ta[1], tb[0], tb[1]};
+  }
   // EXT compiles the articulated angular block in (the solve kernel's EXT instance, launched for
   // batches with a scene that has it or the contact-then-internal schedule); the EXT = false kernel
   // is the plain contact loop.
@@ -457,29 +500,9 @@ struct SolverT {
         // friction patches only the region's first anchor carries them, with the pooled load.
         const float4 g = rows[o + 19u];
         const bool aon = !ell && (S.PATCH == 0u || role == 1.0f || (role == 2.0f && rows[o + PO + 1u].w == 0.0f));
-        const float nl2 = pooled;
         if (aon && (g.x > 0.0f || g.y > 0.0f)) {
-          const float4 la = rows[o + 21u];
-          const f3 wrel = tb[1] - ta[1];
-          const float ns = clmp(la.x - dot(n, wrel) * g.z, (-g.x) * nl2, g.x * nl2);
-          const float ds = ns - la.x;
-          ta[0] += v3(rows[o + 22u]) * ds; ta[1] += v3(rows[o + 23u]) * ds;
-          tb[0] += v3(rows[o + 24u]) * ds; tb[1] += v3(rows[o + 25u]) * ds;
-          const f3 w2 = tb[1] - ta[1];
-          const float4 ri = rows[o + 20u];
-          const float u1 = dot(t1, w2), u2 = dot(t2, w2);
-          f2 lr = mf2(la.y, la.z) - mf2(ri.x * u1 + ri.y * u2, ri.y * u1 + ri.z * u2);
-          const float rl = g.y * nl2;
-          if (len(lr) > rl) lr = lr * (rl / fmx(len(lr), 1e-12f));
-          const float d1 = lr.x - la.y, d2 = lr.y - la.z;
-          ta[0] += v3(rows[o + 26u]) * d1 + v3(rows[o + 30u]) * d2;
-          ta[1] += v3(rows[o + 27u]) * d1 + v3(rows[o + 31u]) * d2;
-          tb[0] += v3(rows[o + 28u]) * d1 + v3(rows[o + 32u]) * d2;
-          tb[1] += v3(rows[o + 29u]) * d1 + v3(rows[o + 33u]) * d2;
-          rows[o + 21u] = make_float4(ns, lr.x, lr.y, 0.0f);
-          const f3 tq = (n * ds + t1 * d1) + t2 * d2;
-          add_imp(a, sp3(0.0f), -tq);
-          add_imp(b, sp3(0.0f), tq);
+          const Twists r = free_angular(row, a, b, n, t1, t2, pooled, ta[0], ta[1], tb[0], tb[1]);
+          ta[0] = r.ta0; ta[1] = r.ta1; tb[0] = r.tb0; tb[1] = r.tb1;
         }
       }
       if (S.TORS == 1u && row == S.sched[S.S_UTP + us]) torsion(us, a, b, it, ta, tb);
@@ -493,6 +516,309 @@ struct SolverT {
     solve_row<EXT>(f2u(sl.y), f2u(sl.x), f2i(sl.z), f2i(sl.w), mode, it);
   }
 
+
+  // --- packed rows ---------------------------------------------------------------------------
+  // A contact row is visited 13 times per substep by one thread, in color order. The row records
+  // (23 float4 at a stride of 368 B, in contact order) make a warp's load of one field touch 32
+  // lines and come in many dependent steps: a color of a single warp took 5,700 cycles on 12 boxes.
+  // So once per solve the rows are packed color by color into tiles of 8 rows, field by field (a
+  // field of a tile is one 128 B line, every field at a constant offset from the row's address), in
+  // shared memory when the scene's rows fit, else in global memory.
+  //   0 n, 1/K      1 ra, rhs      2 rb, weight   3 impulses, anchor bound (updated by every visit)
+  //   4 bodies, row and flags, unit, mu           5 t1    6 t2, scale
+  //   7 friction block (largest, smallest, eigenvector)   8 fra, bias 1   9 frb, bias 2
+  //   10-14 the angular responses of both bodies and 1/m of each
+  // The linear response of a free body is its direction over its mass, so it is not stored; a link's
+  // is read from the row record. What a visit does not change (the friction block's eigenvalues and
+  // eigenvector, the anchor bias) is computed here with the operations the visit would use.
+  // About 70% of the visits are of contacts that are near but not touching and change nothing: such
+  // a visit stops after the normal impulse, having read the first five fields.
+  // Scenes with the coupled friction modes, articulated torsion or cone friction, compliance,
+  // momentum or a velocity pass keep the row records (solve_row).
+  enum : uint32_t {
+    PKF_LA = 1u, PKF_LB = 2u,       // the side is a link (linear response in the row record)
+    PKF_IA = 4u, PKF_IB = 8u,       // the side collects link impulses (kind 2)
+    PKF_FRIC = 16u,                 // the row has friction (not a patch member)
+    PKF_UNIT = 32u,                 // its impulse counts in the load of its unit of several rows
+    PKF_POOL = 64u,                 // its friction bound is the unit's pooled load (patch anchor)
+    PKF_FINITE = 128u,              // a zero impulse times its responses is zero, not NaN
+    PKF_ANG = 256u                  // it carries the free bodies' spin and rolling rows
+  };
+  static constexpr uint32_t PKF_SHIFT = 23u;  // row index below, flags above
+  char* pk;              // packed rows: PK_TILE bytes per tile (shared or global)
+  const uint32_t* pkc;   // team launches with rows in shared memory: this block's first chunk of each color
+  __device__ bool packed() const {
+    return S.FMODE == 0u && S.ANG_ART == 0u && S.TORS == 0u && S.NEST == 0u && S.COMPL == 0u && S.VELITERS == 0u &&
+           S.MAXC <= (1u << PKF_SHIFT);
+  }
+  // Address of row i of color c in the global layout: color c's tiles start at (its first slot) / 8
+  // + c, which leaves each color room for its partly filled last tile.
+  static __device__ size_t pk_offset(const uint32_t* wcs, uint32_t c, uint32_t i) {
+    return (size_t)((wcs[c] >> 3u) + c + (i >> 3u)) * PK_TILE + (i & 7u) * 16u;
+  }
+  // In a team launch a block keeps its own chunks of 32 rows (chunk j of a color belongs to block
+  // j mod grid, Team<true>::rank), color after color.
+  __device__ char* pk_at(const uint32_t* wcs, uint32_t c, uint32_t i) const {
+    if (TEAM && pkc != nullptr)
+      return pk + (size_t)(pkc[c] + (i >> 5u) / gridDim.x) * (4u * PK_TILE) + ((i >> 3u) & 3u) * PK_TILE + (i & 7u) * 16u;
+    return pk + pk_offset(wcs, c, i);
+  }
+  static __device__ float4& pf(char* p, uint32_t f) { return *reinterpret_cast<float4*>(p + f * 128u); }
+  __device__ void pack_row(char* p, uint32_t row, uint32_t us, uint32_t key) const {
+    const float4* R = S.rows + (size_t)row * S.ROWS;
+    const int a = (int)(key & 0xffffu) - 1, b = (int)(key >> 16u) - 1;
+    uint32_t fl = 0u;
+    float ima = 0.0f, imb = 0.0f;
+    if (a >= 0) {
+      const uint32_t k = bkind(a);
+      if (k == 1u) ima = S.sf[S.SF_BODY + (uint32_t)a * 8u].x; else fl |= PKF_LA;
+      if (k == 2u) fl |= PKF_IA;
+    }
+    if (b >= 0) {
+      const uint32_t k = bkind(b);
+      if (k == 1u) imb = S.sf[S.SF_BODY + (uint32_t)b * 8u].x; else fl |= PKF_LB;
+      if (k == 2u) fl |= PKF_IB;
+    }
+    const float4 r0 = R[0], r1 = R[1], r2 = R[2], r3 = R[3], r4 = R[4], ki = R[5], lam = R[6];
+    f3 fra = v3(r3), frb = v3(r4);
+    f2 bias = mf2(0.0f, 0.0f);
+    float role = 1.0f, lim = 0.0f;
+    bool first = false;
+    if (S.EXTRA == 1u) {
+      const float4 p0 = R[S.PO], p1 = R[S.PO + 1u], p2 = R[S.PO + 2u];
+      role = p0.w;
+      fra = v3(p0);
+      frb = v3(p1);
+      first = p1.w == 0.0f;
+      lim = p2.w;
+      if (S.PATCH == 1u) {
+        // The pooled load of a unit of one row is that row's impulse: no shared sum needed.
+        const bool several = S.sched[S.S_USIZE + us] > 1u;
+        if (role != 1.0f && several) fl |= PKF_UNIT;
+        S.plam[row] = role != 1.0f ? lam.x : 0.0f;
+        if (role == 2.0f) {
+          fl |= PKF_POOL;
+          const f3 e = v3(p2);
+          bias = (S.F_ANCHOR_BETA * mf2(dot(v3(r1), e), dot(v3(r2), e))) / P.dt;
+        }
+      }
+    }
+    if (role != 0.0f) fl |= PKF_FRIC;
+    if (S.ANG == 1u) {
+      const float4 g = R[19];
+      if ((S.PATCH == 0u || role == 1.0f || (role == 2.0f && first)) && (g.x > 0.0f || g.y > 0.0f)) fl |= PKF_ANG;
+    }
+    const float kd = ki.x * ki.z - ki.y * ki.y;
+    const FricEig e = fric_eig(ki.z / kd, -ki.y / kd, ki.x / kd);
+    f3 ma[3], mb[3];
+    float fin = ((r0.x + r0.y) + r0.z) * 0.0f + ((r3.x + r3.y) + r3.z) * 0.0f + ((r4.x + r4.y) + r4.z) * 0.0f;
+#pragma unroll
+    for (uint32_t r = 0; r < 3u; r++) {
+      const float4 la = R[7u + r * 4u], aa = R[8u + r * 4u], lb = R[9u + r * 4u], ab = R[10u + r * 4u];
+      ma[r] = v3(aa);
+      mb[r] = v3(ab);
+      fin += ((la.x * 0.0f + la.y * 0.0f) + la.z * 0.0f) + ((aa.x * 0.0f + aa.y * 0.0f) + aa.z * 0.0f);
+      fin += ((lb.x * 0.0f + lb.y * 0.0f) + lb.z * 0.0f) + ((ab.x * 0.0f + ab.y * 0.0f) + ab.z * 0.0f);
+    }
+    if (fin == 0.0f) fl |= PKF_FINITE;
+    pf(p, 0) = r0;
+    pf(p, 1) = mf4(v3(r3), r1.w);
+    pf(p, 2) = mf4(v3(r4), ki.w);
+    pf(p, 3) = mf4(v3(lam), lim);
+    pf(p, 4) = make_float4(__uint_as_float(key), __uint_as_float(row | (fl << PKF_SHIFT)), __uint_as_float(us), r2.w);
+    pf(p, 5) = mf4(v3(r1), 0.0f);
+    pf(p, 6) = mf4(v3(r2), e.scale);
+    pf(p, 7) = make_float4(e.largest, e.smallest, e.vx, e.vy);
+    pf(p, 8) = mf4(fra, bias.x);
+    pf(p, 9) = mf4(frb, bias.y);
+    pf(p, 10) = mf4(ma[0], ima);
+    pf(p, 11) = mf4(mb[0], imb);
+    pf(p, 12) = mf4(ma[1], ma[2].x);
+    pf(p, 13) = make_float4(ma[2].y, ma[2].z, mb[1].x, mb[1].y);
+    pf(p, 14) = mf4(mb[1].z, mb[2]);
+  }
+  // The impulses and anchor bounds back into the row record (warm table, anchors, readers).
+  __device__ void unpack_row(char* p) const {
+    const float4 lam = pf(p, 3), m = pf(p, 4);
+    const uint32_t rf = __float_as_uint(m.y);
+    float4* R = S.rows + (size_t)(rf & ((1u << PKF_SHIFT) - 1u)) * S.ROWS;
+    R[6] = mf4(v3(lam), R[6].w);
+    if (((rf >> PKF_SHIFT) & PKF_POOL) != 0u) R[S.PO + 2u].w = lam.w;
+  }
+  // What every visit reads; loaded for a thread's next row before the barrier of the current color
+  // (only the row's own thread changes its impulses).
+  struct PkHead { float4 f0, f1, f2, f3, m; };
+  static __device__ PkHead pk_load(char* p) { return PkHead{pf(p, 0), pf(p, 1), pf(p, 2), pf(p, 3), pf(p, 4)}; }
+  // Adding a zero changes only a component that is -0, the least word among the components as
+  // signed integers.
+  static __device__ bool minus_zero(f3 x, f3 y) {
+    const int m = min(min(__float_as_int(x.x), min(__float_as_int(x.y), __float_as_int(x.z))),
+                      min(__float_as_int(y.x), min(__float_as_int(y.y), __float_as_int(y.z))));
+    return m == (int)0x80000000;
+  }
+  __device__ void add_link_imp(int b, f3 f, f3 t) const {
+    imp[(uint32_t)b * 2u] = add4(imp[(uint32_t)b * 2u], mf4(f, 0.0f));
+    imp[(uint32_t)b * 2u + 1u] = add4(imp[(uint32_t)b * 2u + 1u], mf4(t, 0.0f));
+  }
+  struct PkBody { float4 f5, f6, f7, f8, f9, f10, f11; };
+  static __device__ PkBody pk_body(char* p) {
+    return PkBody{pf(p, 5), pf(p, 6), pf(p, 7), pf(p, 8), pf(p, 9), pf(p, 10), pf(p, 11)};
+  }
+  // One visit of the row at p: solve_row's operations in its order (WARM: the warm impulses of the
+  // sweep before the first; else a solve. ANG: the scene has free bodies' spin and rolling rows).
+  template <bool WARM, bool ANG>
+  __device__ __forceinline__ void solve_packed(char* p, const PkHead& h, uint32_t it, float omega, float* uload) const {
+    const uint32_t key = __float_as_uint(h.m.x), rf = __float_as_uint(h.m.y), fl = rf >> PKF_SHIFT;
+    const uint32_t row = rf & ((1u << PKF_SHIFT) - 1u), us = __float_as_uint(h.m.z);
+    const int a = (int)(key & 0xffffu) - 1, b = (int)(key >> 16u) - 1;
+    f3 ta0 = sp3(0.0f), ta1 = ta0, tb0 = ta0, tb1 = ta0;
+    if (a >= 0) { ta0 = v3(tw[2 * a]); ta1 = v3(tw[2 * a + 1]); }
+    if (b >= 0) { tb0 = v3(tw[2 * b]); tb1 = v3(tw[2 * b + 1]); }
+    float load = 0.0f;
+    if (!WARM && (fl & PKF_UNIT) != 0u) load = uload[us];
+    float4 lam = h.f3;
+    const f3 n = v3(h.f0), ra = v3(h.f1), rb = v3(h.f2);
+    float dn = lam.x;
+    bool fric = true;
+    float lim = 0.0f, pooled = 0.0f;
+    if (WARM) {
+      if (lam.x == 0.0f && lam.y == 0.0f && lam.z == 0.0f && (fl & PKF_FINITE) != 0u && !minus_zero(ta0, ta1) && !minus_zero(tb0, tb1)) return;
+    } else {
+      const f3 vrel = (tb0 + cross(tb1, rb)) - (ta0 + cross(ta1, ra));
+      const float jv = dot(n, vrel);
+      const float w = h.f2.w;
+      const float res = jv + h.f1.w;
+      const float nl = fmx(lam.x + omega * ((((-res) * h.f0.w) * w) - (1.0f - w) * lam.x), 0.0f);
+      dn = nl - lam.x;
+      const bool same = __float_as_uint(nl) == __float_as_uint(lam.x) && __float_as_uint(dn) == 0u;
+      // The friction bound: the row's own normal impulse, or the unit's pooled load at a patch
+      // anchor (0 + the impulses of its rows, as the load pass sums them).
+      pooled = nl;
+      if ((fl & (PKF_UNIT | PKF_POOL)) != 0u) {
+        if ((fl & PKF_UNIT) != 0u) {
+          load += dn;
+          if (!same) { uload[us] = load; S.plam[row] = nl; }
+        } else {
+          load = (0.0f + lam.x) + dn;
+        }
+        if ((fl & PKF_POOL) != 0u) pooled = load;
+      }
+      lim = h.m.w * pooled;
+      fric = (fl & PKF_FRIC) != 0u && it >= S.FSTART;
+      const bool flat = (__float_as_uint(lam.y) | __float_as_uint(lam.z)) == 0u;
+      lam.x = nl;
+      if ((fl & PKF_POOL) != 0u) lam.w = lim;
+      if (same && (flat || !(fric || it < S.FSTART)) && (!fric || lim <= 0.0f) && (fl & (PKF_FINITE | (ANG ? PKF_ANG : 0u))) == PKF_FINITE &&
+          !minus_zero(ta0, ta1) && !minus_zero(tb0, tb1)) {
+        if (__float_as_uint(lam.w) != __float_as_uint(h.f3.w)) pf(p, 3) = lam;
+        return;
+      }
+    }
+    const PkBody B = pk_body(p);
+    const f3 t1 = v3(B.f5), t2 = v3(B.f6), fra = v3(B.f8), frb = v3(B.f9);
+    // The tangential responses' loads are in flight during the friction solve.
+    const float4 f12 = pf(p, 12), f13 = pf(p, 13), f14 = pf(p, 14);
+    const bool linked = (fl & (PKF_LA | PKF_LB)) != 0u;
+    const float4* R = S.rows + (size_t)row * S.ROWS;
+    const float ima = B.f10.w, imb = B.f11.w;
+    {
+      f3 la = (-n) * ima, lb = n * imb;  // linear responses of n
+      if (linked) {
+        if ((fl & PKF_LA) != 0u) la = v3(R[7]);
+        if ((fl & PKF_LB) != 0u) lb = v3(R[9]);
+      }
+      ta0 += la * dn; ta1 += v3(B.f10) * dn;
+      tb0 += lb * dn; tb1 += v3(B.f11) * dn;
+    }
+    if (!WARM && (fl & (PKF_IA | PKF_IB)) != 0u) {
+      if ((fl & PKF_IA) != 0u) add_link_imp(a, -n * dn, -cross(v3(pf(p, 1)), n * dn));
+      if ((fl & PKF_IB) != 0u) add_link_imp(b, n * dn, cross(v3(pf(p, 2)), n * dn));
+    }
+    float dt1 = lam.y, dt2 = lam.z;
+    if (!WARM) {
+      if (it < S.FSTART) { lam.y = 0.0f; lam.z = 0.0f; }
+      if (fric) {
+        f2 lt = mf2(0.0f, 0.0f);  // a zero bound: no tangential velocities needed
+        if (!(lim <= 0.0f)) {
+          const f3 vr2 = (tb0 + cross(tb1, frb)) - (ta0 + cross(ta1, fra));
+          const float v1 = dot(t1, vr2) + B.f8.w, v2_ = dot(t2, vr2) + B.f9.w;
+          lt = fric_solve(FricEig{B.f6.w, B.f7.x, B.f7.y, B.f7.z, B.f7.w}, v1, v2_, lam.y, lam.z, lim, omega);
+        }
+        dt1 = lt.x - lam.y;
+        dt2 = lt.y - lam.z;
+        lam.y = lt.x;
+        lam.z = lt.y;
+      }
+      pf(p, 3) = lam;
+    }
+    if (fric) {
+      f3 la1 = (-t1) * ima, la2 = (-t2) * ima, lb1 = t1 * imb, lb2 = t2 * imb;  // of t1 and t2
+      if (linked) {
+        if ((fl & PKF_LA) != 0u) { la1 = v3(R[11]); la2 = v3(R[15]); }
+        if ((fl & PKF_LB) != 0u) { lb1 = v3(R[13]); lb2 = v3(R[17]); }
+      }
+      const f3 a1 = v3(f12), a2 = mf3(f12.w, f13.x, f13.y), b1 = mf3(f13.z, f13.w, f14.x), b2 = mf3(f14.y, f14.z, f14.w);
+      if (WARM) {
+        ta0 += la1 * dt1; ta1 += a1 * dt1;
+        tb0 += lb1 * dt1; tb1 += b1 * dt1;
+        ta0 += la2 * dt2; ta1 += a2 * dt2;
+        tb0 += lb2 * dt2; tb1 += b2 * dt2;
+      } else {
+        ta0 += la1 * dt1 + la2 * dt2;
+        ta1 += a1 * dt1 + a2 * dt2;
+        tb0 += lb1 * dt1 + lb2 * dt2;
+        tb1 += b1 * dt1 + b2 * dt2;
+      }
+      if ((fl & (PKF_IA | PKF_IB)) != 0u) {
+        const f3 ft = t1 * dt1 + t2 * dt2;
+        if (WARM) {
+          const f3 fn_ = n * dn;
+          if ((fl & PKF_IA) != 0u) add_link_imp(a, -fn_ - ft, -cross(ra, fn_) - cross(fra, ft));
+          if ((fl & PKF_IB) != 0u) add_link_imp(b, fn_ + ft, cross(rb, fn_) + cross(frb, ft));
+        } else {
+          if ((fl & PKF_IA) != 0u) add_link_imp(a, -ft, -cross(fra, ft));
+          if ((fl & PKF_IB) != 0u) add_link_imp(b, ft, cross(frb, ft));
+        }
+      }
+    }
+    if (ANG && (fl & PKF_ANG) != 0u) {
+      const Twists r = free_angular(row, a, b, n, t1, t2, pooled, ta0, ta1, tb0, tb1);
+      ta0 = r.ta0; ta1 = r.ta1; tb0 = r.tb0; tb1 = r.tb1;
+    }
+    if (a >= 0) { tw[2 * a] = mf4(ta0, 0.0f); tw[2 * a + 1] = mf4(ta1, 0.0f); }
+    if (b >= 0) { tw[2 * b] = mf4(tb0, 0.0f); tw[2 * b + 1] = mf4(tb1, 0.0f); }
+  }
+  // The rows of one sweep, color by color, then the overflow color in contact order by one thread.
+  template <bool WARM, bool ANG>
+  __device__ __forceinline__ void packed_sweep(uint32_t ncol, uint32_t it, const uint32_t* wcs) const {
+    const uint32_t tid = tm.rank(), nt = tm.size();
+    const float omega = S.F_OMEGA;
+    float* uload = S.art + S.A_ULOAD;
+    PkHead h;
+    bool ready = false;
+    uint32_t s0 = ncol > 0u ? wcs[0] : 0u;
+    for (uint32_t c = 0; c < ncol; c++) {
+      const uint32_t s1 = wcs[c + 1u];
+      for (uint32_t i = tid; i < s1 - s0; i += nt) {
+        char* p = pk_at(wcs, c, i);
+        if (!ready) h = pk_load(p);
+        ready = false;
+        solve_packed<WARM, ANG>(p, h, it, omega, uload);
+      }
+      if (c + 1u < ncol && tid < wcs[c + 2u] - s1) {
+        h = pk_load(pk_at(wcs, c + 1u, tid));
+        ready = true;
+      }
+      s0 = s1;
+      tm.sync();
+    }
+    const uint32_t nover = wcs[S.NCOL + 1u] - wcs[S.NCOL];
+    if (tid == 0u)
+      for (uint32_t i = 0; i < nover; i++) {
+        char* p = S.pk + pk_offset(wcs, S.NCOL, i);
+        solve_packed<WARM, ANG>(p, pk_load(p), it, omega, uload);
+      }
+  }
 
   // subgroupAdd over the warp (wgsl.js:3305, subgroups on), pinned to an xor butterfly over lane
   // offsets 16, 8, 4, 2, 1. IEEE addition commutes, so every lane ends with the same bits.
@@ -944,12 +1270,14 @@ struct SolverT {
   }
   // One sweep (wgsl.js:3559-3611).
   template <bool EXT>
+  // Inline: a separate function's calling convention spilled the packed rows' registers (568 bytes).
   // ph: 0 every row; 1 contacts only (no joint-internal rows, no velocity-limit rows, no internal
   // dense rows); 2 joint-internal rows only (no contact slots, no contact dense rows). The two
   // partial sweeps serve row_schedule "contact_then_internal" (wgsl.js:3559-3590).
-  __device__ void sweep(uint32_t mode, uint32_t ncol0, uint32_t it, const uint32_t* wcs, uint32_t nu, uint32_t ph) const {
+  __device__ __forceinline__ void sweep(uint32_t mode, uint32_t ncol0, uint32_t it, const uint32_t* wcs, uint32_t nu, uint32_t ph) const {
     const uint32_t tid = tm.rank(), nt = tm.size();
     const uint32_t ncol = ph == 2u ? 0u : ncol0;
+    const bool pk_on = packed();
     if (ph != 1u)
       for (uint32_t a = tid; a < S.NA; a += nt) joint_rows(a);
     if (S.PATCH == 1u && mode == 1u) {
@@ -968,22 +1296,34 @@ struct SolverT {
 #pragma unroll
         for (uint32_t k = 0; k < UL; k++) {
           load[k] = 0.0f;
-          for (uint32_t m = s0[k]; m < s0[k] + n[k]; m++)
-            if (S.rows[m * S.ROWS + S.PO].w != 1.0f) load[k] += S.rows[m * S.ROWS + 6u].x;
+          if (pk_on && n[k] < 2u) continue;  // a packed row alone in its unit is its own load
+          if (pk_on)
+            for (uint32_t m = s0[k]; m < s0[k] + n[k]; m++) load[k] += S.plam[m];  // 0 outside the patch
+          else
+            for (uint32_t m = s0[k]; m < s0[k] + n[k]; m++)
+              if (S.rows[m * S.ROWS + S.PO].w != 1.0f) load[k] += S.rows[m * S.ROWS + 6u].x;
         }
 #pragma unroll
         for (uint32_t k = 0; k < UL; k++)
-          if (us0 + k * nt < nu) S.art[S.A_ULOAD + us0 + k * nt] = load[k];
+          if (us0 + k * nt < nu && !(pk_on && n[k] < 2u)) S.art[S.A_ULOAD + us0 + k * nt] = load[k];
       }
     }
     tm.sync();
     dense_phase(1u, it, ph);
-    for (uint32_t c = 0; c < ncol; c++) {
-      for (uint32_t u = wcs[c] + tid; u < wcs[c + 1u]; u += nt) solve_slot<EXT>(u, mode, it);
-      tm.sync();
+    if (pk_on) {
+      if (ph != 2u) {
+        if (mode == 0u) packed_sweep<true, false>(ncol, it, wcs);
+        else if (S.ANG == 1u) packed_sweep<false, true>(ncol, it, wcs);
+        else packed_sweep<false, false>(ncol, it, wcs);
+      }
+    } else {
+      for (uint32_t c = 0; c < ncol; c++) {
+        for (uint32_t u = wcs[c] + tid; u < wcs[c + 1u]; u += nt) solve_slot<EXT>(u, mode, it);
+        tm.sync();
+      }
+      if (tid == 0u && ph != 2u)
+        for (uint32_t u = wcs[S.NCOL]; u < wcs[S.NCOL + 1u]; u++) solve_slot<EXT>(u, mode, it);
     }
-    if (tid == 0u && ph != 2u)
-      for (uint32_t u = wcs[S.NCOL]; u < wcs[S.NCOL + 1u]; u++) solve_slot<EXT>(u, mode, it);
     tm.sync();
     for (uint32_t a = tid; a < S.NA; a += nt) {
       contact_impulses(a);
@@ -1118,9 +1458,25 @@ __device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team
   for (uint32_t i = tid; i < 2u * S.ND; i += nt) A[S.A_LIM + i] = 0.0f;
   for (uint32_t i = tid; i < S.ND; i += nt) { A[S.A_FRIC + i] = 0.0f; A[S.A_DRV + i] = 0.0f; }
   const uint32_t nslot = wcs[S.NCOL + 1u];
+  const bool pk_on = sv.packed();
+  // Packed rows in shared memory when they fit what the launch has beyond the scene's staging: the
+  // whole scene's, or in a team launch this block's chunks (copied from the global layout below).
+  char* pk_global = reinterpret_cast<char*>(S.pk);
+  char* rows_sm = reinterpret_cast<char*>(sb) + ((lay.total + 127u) & ~127u);
+  const uint32_t rows_room = B.solve_smem > ((lay.total + 127u) & ~127u) ? B.solve_smem - ((lay.total + 127u) & ~127u) : 0u;
+  const uint32_t ncs = wcs[ncol];  // rows of the colors, without the overflow color's
+  bool rows_shared = pk_on && !TEAM && ((size_t)(ncs >> 3u) + ncol + 1u) * PK_TILE <= rows_room;
+  sv.pk = rows_shared ? rows_sm : pk_global;
+  sv.pkc = nullptr;
   for (uint32_t u = tid; u < nslot; u += nt) {
     uint32_t row = S.sched[S.S_PORD + u], us = S.sched[S.S_RUNIT + row], key = S.sched[S.S_UKEY + us];
     S.slots[2u * u] = make_float4((float)row, (float)us, (float)((int)(key & 0xffffu) - 1), (float)((int)(key >> 16u) - 1));
+    if (pk_on) {
+      const uint32_t c = S.sched[S.S_PCOL + row];
+      // The overflow color stays in global memory (one thread runs it, whichever layout the colors have).
+      const size_t o = SolverT<TEAM>::pk_offset(wcs, c, u - wcs[c]);
+      sv.pack_row((rows_shared && !TEAM && c < ncol ? rows_sm : pk_global) + o, row, us, key);
+    }
   }
   tm.sync();
   // Few articulations: a warp each (the chain recursion shortened); many: a thread each.
@@ -1136,22 +1492,9 @@ __device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team
     if (!TEAM || blockIdx.x == 0u) sv.dense_lists(dtmp);
     if (TEAM) tm.sync();
   }
-  sv.dense_phase(0u, 0u, 0u);
-  sv.sweep<EXT>(0u, ncol, 0u, wcs, nu, 0u);
-  // row_schedule "contact_then_internal" (wgsl.js:3693-3696): all contact iterations (phase 1),
-  // then the joint-internal rows (phase 2); otherwise one pass of full sweeps (phase 0).
-  // Only the EXT instance carries it.
-  const bool cti = EXT && S.CTI == 1u;
-  const uint32_t npass = cti ? 2u : 1u;
-  for (uint32_t pass = 0; pass < npass; pass++)
-    for (uint32_t it = 0; it < P.iterations; it++) {
-      // Nesterov momentum keeps block-wide sums: a team launch is never made for a scene with it.
-      if (!TEAM && S.NEST == 1u && pass == 0u) sv.momentum_step(ncol, it, wcs);
-      sv.sweep<EXT>(1u, ncol, it, wcs, nu, cti ? pass + 1u : 0u);
-    }
   // Velocity pass (velocity_iterations, wgsl.js:3700-3736): positions integrate with the velocities
   // reached here; further bias-free sweeps from the accumulated impulses set the output velocities.
-  if (S.VELITERS > 0u) {
+  auto velocity_snapshot = [&]() {
     for (uint32_t b = tid; b < S.NB; b += nt) {
       sv.ar.ast3(S.A_SNAP + b * 8u, v3(sv.tw[b * 2u]));
       sv.ar.ast3(S.A_SNAP + b * 8u + 4u, v3(sv.tw[b * 2u + 1u]));
@@ -1186,8 +1529,36 @@ __device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team
     }
     tm.sync();
     sv.vpass = true;
-    for (uint32_t it = 0; it < S.VELITERS; it++) sv.sweep<EXT>(1u, ncol, P.iterations + it, wcs, nu, 0u);
-    sv.vpass = false;
+  };
+  sv.dense_phase(0u, 0u, 0u);
+  // The warm-apply sweep, the iterations and the velocity pass's sweeps, from one place (so the
+  // sweep is compiled once, inline). row_schedule "contact_then_internal" (wgsl.js:3693-3696): all
+  // contact iterations (phase 1), then the joint-internal rows (phase 2); otherwise one pass of full
+  // sweeps (phase 0). Only the EXT instance carries it.
+  const bool cti = EXT && S.CTI == 1u;
+  const uint32_t npos = (cti ? 2u : 1u) * P.iterations;
+  for (uint32_t k = 0; k <= npos + S.VELITERS; k++) {
+    uint32_t it = 0u, ph = 0u;
+    if (k > npos) {
+      if (k == npos + 1u) velocity_snapshot();
+      it = P.iterations + (k - npos - 1u);
+    } else if (k > 0u) {
+      const bool second = k > P.iterations;
+      it = k - 1u - (second ? P.iterations : 0u);
+      if (cti) ph = second ? 2u : 1u;
+      // Nesterov momentum keeps block-wide sums: a team launch is never made for a scene with it.
+      if (!TEAM && S.NEST == 1u && !second) sv.momentum_step(ncol, it, wcs);
+    }
+    sv.template sweep<EXT>(k == 0u ? 0u : 1u, ncol, it, wcs, nu, ph);
+  }
+  sv.vpass = false;
+  if (pk_on) {
+    for (uint32_t u = tid; u < nslot; u += nt) {
+      const uint32_t c = S.sched[S.S_PCOL + S.sched[S.S_PORD + u]];
+      const size_t o = SolverT<TEAM>::pk_offset(wcs, c, u - wcs[c]);
+      sv.unpack_row((c < ncol ? sv.pk : pk_global) + o);
+    }
+    tm.sync();
   }
   // Warm-start table (wgsl.js:3737-3767): rows sharing a key keep the largest normal impulse.
   const uint32_t nc = S.sched[S.S_USTART + nu];
