@@ -96,6 +96,8 @@ struct SceneHost {
   size_t o_rkeys1 = 0, o_rstat = 0, o_rhist = 0, o_rctr = 0;
   size_t art_floats = 0, sched_words = 0, warm_words = 0, tscr_floats = 0;
   std::vector<float> statF;
+  std::vector<uint32_t> levels;  // SceneDev::lt
+  size_t o_lt = 0, o_dhd = 0;
   std::vector<uint32_t> statU;
   std::vector<float4> pos0, rot0, lv0, av0;
   std::vector<float> art0;
@@ -177,6 +179,47 @@ struct steel_batch {
 
 namespace {
 
+// The articulation trees by level (SceneDev::lt), from the packed link records.
+void build_levels(SceneHost& s) {
+  SceneDev& d = s.d;
+  const uint32_t NA = d.NA, NL = d.NL;
+  auto parent = [&](uint32_t l) { return (int)s.statF[4u * (d.SF_LINK + l * 6u) + 1u]; };
+  std::vector<uint32_t> depth(NL, 0u), lvb(NA + 1u, 0u), lvo{0u}, lvl, chs(NL + 1u, 0u), chl;
+  for (uint32_t l = 0; l < NL; l++) {
+    const int p = parent(l);
+    depth[l] = p >= 0 && (uint32_t)p < l ? depth[p] + 1u : 0u;
+  }
+  for (uint32_t a = 0; a < NA; a++) {
+    const uint32_t* ai = s.statU.data() + d.SU_ART + a * 4u;
+    uint32_t top = 0u;
+    for (uint32_t l = ai[0]; l < ai[0] + ai[1]; l++) top = std::max(top, depth[l] + 1u);
+    for (uint32_t k = 0; k < top; k++) {
+      for (uint32_t l = ai[0]; l < ai[0] + ai[1]; l++)
+        if (depth[l] == k) lvl.push_back(l);
+      lvo.push_back((uint32_t)lvl.size());
+    }
+    lvb[a + 1u] = (uint32_t)lvo.size() - 1u;
+  }
+  std::vector<std::vector<uint32_t>> children(NL);
+  for (uint32_t l = NL; l-- > 0u;)
+    if (parent(l) >= 0) children[(uint32_t)parent(l)].push_back(l);
+  for (uint32_t l = 0; l < NL; l++) {
+    chl.insert(chl.end(), children[l].begin(), children[l].end());
+    chs[l + 1u] = (uint32_t)chl.size();
+  }
+  auto add = [&](const std::vector<uint32_t>& v) {
+    const uint32_t o = (uint32_t)s.levels.size();
+    s.levels.insert(s.levels.end(), v.begin(), v.end());
+    return o;
+  };
+  s.levels.clear();
+  add(lvb);
+  d.LT_LVO = add(lvo);
+  d.LT_LVL = add(lvl);
+  d.LT_CHS = add(chs);
+  d.LT_CHL = add(chl);
+}
+
 // threads: the largest prepare / solve block; one_scene: the batch has this scene alone (a team
 // launch may run it, whose scratch passes use TEAM_SCRATCH_BLOCKS blocks' threads).
 int build_scene(SceneHost& s, const steel_scene_desc& in, Layout& L, uint32_t threads, bool one_scene,
@@ -250,6 +293,7 @@ int build_scene(SceneHost& s, const steel_scene_desc& in, Layout& L, uint32_t th
     // parallel coloring: per-body row lists and frontiers, row keys
     put(d.S_BSTART, NB + 1); put(d.S_BPOS, NB); put(d.S_BREADY, NB); put(d.S_BLIST, 2 * (size_t)MAXC);
     put(d.S_RKEY, MAXC); put(d.S_RFLAG, MAXC); put(d.S_WL, 2 * (size_t)NB);
+    put(d.S_DFIN, d.MAXDENSE); put(d.S_DSTATE, NA);
     s.sched_words = so;
   }
   s.warm_words = 10ull * d.WH + 30ull * d.AH;
@@ -262,6 +306,7 @@ int build_scene(SceneHost& s, const steel_scene_desc& in, Layout& L, uint32_t th
   // Host copies: static data and initial state (the reference's reset() contents).
   s.statF.assign(in.statF, in.statF + in.statF_floats);
   s.statU.assign(in.statU, in.statU + in.statU_words);
+  build_levels(s);
   s.pos0.resize(NB); s.rot0.resize(NB); s.lv0.resize(NB); s.av0.resize(NB);
   for (uint32_t b = 0; b < NB; b++) {
     const float* p = in.body_pose + b * 8;
@@ -284,6 +329,7 @@ int build_scene(SceneHost& s, const steel_scene_desc& in, Layout& L, uint32_t th
   const size_t arena0 = L.bytes;
   s.o_sf = L.take(s.statF.size() * 4);
   s.o_su = L.take(s.statU.size() * 4);
+  s.o_lt = L.take(s.levels.size() * 4); s.o_dhd = L.take((size_t)d.MAXDENSE * 32u + 32u);
   s.o_pos = L.take((size_t)NB * 16); s.o_rot = L.take((size_t)NB * 16);
   s.o_ppos = L.take((size_t)NB * 16); s.o_prot = L.take((size_t)NB * 16);
   s.o_lv = L.take((size_t)NB * 16); s.o_av = L.take((size_t)NB * 16);
@@ -734,6 +780,8 @@ int steel_batch_create(steel_ctx* ctx, const steel_scene_desc* scenes, uint32_t 
     SceneDev& d = s.d;
     d.sf = RO<float4>{at<float4>(A, s.o_sf)};
     d.su = RO<uint32_t>{at<uint32_t>(A, s.o_su)};
+    d.lt = RO<uint32_t>{at<uint32_t>(A, s.o_lt)};
+    d.dhd = at<float4>(A, s.o_dhd);
     d.pos = at<float4>(A, s.o_pos); d.rot = at<float4>(A, s.o_rot);
     d.ppos = at<float4>(A, s.o_ppos); d.prot = at<float4>(A, s.o_prot);
     d.lv = at<float4>(A, s.o_lv); d.av = at<float4>(A, s.o_av);
@@ -765,6 +813,7 @@ int steel_batch_create(steel_ctx* ctx, const steel_scene_desc* scenes, uint32_t 
     solve_ext |= d.ANG_ART | d.CTI;
     dev[i] = d;
     CU(cudaMemcpyAsync((void*)d.sf.p, s.statF.data(), s.statF.size() * 4, cudaMemcpyHostToDevice, st));
+    CU(cudaMemcpyAsync((void*)d.lt.p, s.levels.data(), s.levels.size() * 4, cudaMemcpyHostToDevice, st));
     CU(cudaMemcpyAsync((void*)d.su.p, s.statU.data(), s.statU.size() * 4, cudaMemcpyHostToDevice, st));
   }
   BatchDev& bd = b->bd;

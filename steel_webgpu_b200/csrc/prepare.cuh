@@ -620,6 +620,11 @@ struct Prep {
     A[o + 9u] = ln; A[o + 10u] = lt.x; A[o + 11u] = lt.y;
     ar.ast3(o + 12u, t1); ar.ast3(o + 15u, t2); ar.ast3(o + 18u, n);
     A[o + 21u] = 0.0f;
+    // The solve skips the responses of rows without impulse; that is exact when they are finite,
+    // which a finite K implies (each product J Y is a term of it).
+    float kz = 0.0f;
+    for (uint32_t k = 0; k < 9u; k++) kz += K[k] * 0.0f;
+    S.sched[S.S_DFIN + slot] = kz == 0.0f ? 1u : 0u;
     A[o + 24u] = bounce ? 1.0f : row_weight(phi);
     A[o + 22u] = bounce ? 1e30f : phi;
   }

@@ -324,8 +324,9 @@ struct SolverT {
     f3 ta0, ta1, tb0, tb1;
     float l1, l2;
   };
-  __device__ __noinline__ AngOut ang_block(uint32_t o, int a, int b, f3 n, f3 t1, f3 t2, f3 fra, f3 frb, float mu,
-                                           float pooled, float ly, float lz, f3 ta0, f3 ta1, f3 tb0, f3 tb1) const {
+  static __device__ __noinline__ AngOut ang_block(const SolverT sv, uint32_t o, int a, int b, f3 n, f3 t1, f3 t2, f3 fra, f3 frb, float mu,
+                                           float pooled, float ly, float lz, f3 ta0, f3 ta1, f3 tb0, f3 tb1) {
+    const SceneDev& S = sv.S;
     float4* rows = S.rows;
     f3 ta[2] = {ta0, ta1}, tb[2] = {tb0, tb1};
     float H[25];
@@ -354,18 +355,19 @@ struct SolverT {
     tb[1] += (((v3(rows[o + 14u]) * d[0] + v3(rows[o + 18u]) * d[1]) + v3(rows[o + 25u]) * d[2]) + v3(rows[o + 29u]) * d[3]) + v3(rows[o + 33u]) * d[4];
     const f3 f = t1 * d[0] + t2 * d[1];
     const f3 tq = (n * d[2] + t1 * d[3]) + t2 * d[4];
-    add_imp(a, -f, (-cross(fra, f)) - tq);
-    add_imp(b, f, cross(frb, f) + tq);
+    sv.add_imp(a, -f, (-cross(fra, f)) - tq);
+    sv.add_imp(b, f, cross(frb, f) + tq);
     rows[o + 21u] = make_float4(nl5[2], nl5[3], nl5[4], 0.0f);
     return AngOut{ta[0], ta[1], tb[0], tb[1], nl5[0], nl5[1]};
   }
   // A free body's spin and rolling rows of contact row `row` under normal load nl2.
   // Twists go in and out by value, so the caller's stay in registers.
   struct Twists { f3 ta0, ta1, tb0, tb1; };
-  __device__ __noinline__ Twists free_angular(uint32_t row, int a, int b, f3 n, f3 t1, f3 t2, float nl2, f3 ta0, f3 ta1,
-                                              f3 tb0, f3 tb1) const {
+  // (`sv` too: a call through the object's address would keep it in local memory.)
+  static __device__ __noinline__ Twists free_angular(const SolverT sv, uint32_t row, int a, int b, f3 n, f3 t1, f3 t2, float nl2, f3 ta0, f3 ta1,
+                                              f3 tb0, f3 tb1) {
     f3 ta[2] = {ta0, ta1}, tb[2] = {tb0, tb1};
-    float4* R = S.rows + (size_t)row * S.ROWS;
+    float4* R = sv.S.rows + (size_t)row * sv.S.ROWS;
     const float4 g = R[19], la = R[21], ri = R[20];
     const f3 wrel = tb[1] - ta[1];
     const float ns = clmp(la.x - dot(n, wrel) * g.z, (-g.x) * nl2, g.x * nl2);
@@ -384,15 +386,15 @@ struct SolverT {
     tb[1] += v3(R[29]) * d1 + v3(R[33]) * d2;
     R[21] = make_float4(ns, lr.x, lr.y, 0.0f);
     const f3 tq = (n * ds + t1 * d1) + t2 * d2;
-    add_imp(a, sp3(0.0f), -tq);
-    add_imp(b, sp3(0.0f), tq);
+    sv.add_imp(a, sp3(0.0f), -tq);
+    sv.add_imp(b, sp3(0.0f), tq);
     return Twists{ta[0], ta[1], tb[0], tb[1]};
   }
   // EXT compiles the articulated angular block in (the solve kernel's EXT instance, launched for
   // batches with a scene that has it or the contact-then-internal schedule); the EXT = false kernel
   // is the plain contact loop.
   template <bool EXT>
-  __device__ void solve_row(uint32_t us, uint32_t row, int a, int b, uint32_t mode, uint32_t it) const {
+  __device__ __forceinline__ void solve_row(uint32_t us, uint32_t row, int a, int b, uint32_t mode, uint32_t it) const {
     const uint32_t ROWS = S.ROWS, PO = S.PO;
     float4* rows = S.rows;
     f3 ta[2], tb[2];
@@ -489,7 +491,7 @@ struct SolverT {
       const bool art_u = (a >= 0 && bkind(a) >= 2u) || (b >= 0 && bkind(b) >= 2u);
       const bool ell = EXT && S.ANG_ART == 1u && S.ANG == 1u && art_u && (rows[o + 19u].x > 0.0f || rows[o + 19u].y > 0.0f);
       if (ell && it >= S.FSTART) {
-        const AngOut r = ang_block(o, a, b, n, t1, t2, fra, frb, r2.w, pooled, lam.y, lam.z, ta[0], ta[1], tb[0], tb[1]);
+        const AngOut r = ang_block(*this, o, a, b, n, t1, t2, fra, frb, r2.w, pooled, lam.y, lam.z, ta[0], ta[1], tb[0], tb[1]);
         ta[0] = r.ta0; ta[1] = r.ta1; tb[0] = r.tb0; tb[1] = r.tb1;
         lam.y = r.l1;
         lam.z = r.l2;
@@ -501,7 +503,7 @@ struct SolverT {
         const float4 g = rows[o + 19u];
         const bool aon = !ell && (S.PATCH == 0u || role == 1.0f || (role == 2.0f && rows[o + PO + 1u].w == 0.0f));
         if (aon && (g.x > 0.0f || g.y > 0.0f)) {
-          const Twists r = free_angular(row, a, b, n, t1, t2, pooled, ta[0], ta[1], tb[0], tb[1]);
+          const Twists r = free_angular(*this, row, a, b, n, t1, t2, pooled, ta[0], ta[1], tb[0], tb[1]);
           ta[0] = r.ta0; ta[1] = r.ta1; tb[0] = r.tb0; tb[1] = r.tb1;
         }
       }
@@ -510,12 +512,18 @@ struct SolverT {
     if (a >= 0) { tw[(uint32_t)a * 2u] = mf4(ta[0], 0.0f); tw[(uint32_t)a * 2u + 1u] = mf4(ta[1], 0.0f); }
     if (b >= 0) { tw[(uint32_t)b * 2u] = mf4(tb[0], 0.0f); tw[(uint32_t)b * 2u + 1u] = mf4(tb[1], 0.0f); }
   }
+  // The EXT contact loop is a function (by value, as free_angular), so its cone code's frame and
+  // registers stay out of the solve loop.
+  static __device__ __noinline__ void solve_row_ext(const SolverT sv, uint32_t us, uint32_t row, int a, int b,
+                                                    uint32_t mode, uint32_t it) {
+    sv.template solve_row<true>(us, row, a, b, mode, it);
+  }
   template <bool EXT>
   __device__ void solve_slot(uint32_t u, uint32_t mode, uint32_t it) const {
     float4 sl = S.slots[2u * u];
-    solve_row<EXT>(f2u(sl.y), f2u(sl.x), f2i(sl.z), f2i(sl.w), mode, it);
+    if (EXT) solve_row_ext(*this, f2u(sl.y), f2u(sl.x), f2i(sl.z), f2i(sl.w), mode, it);
+    else solve_row<EXT>(f2u(sl.y), f2u(sl.x), f2i(sl.z), f2i(sl.w), mode, it);
   }
-
 
   // --- packed rows ---------------------------------------------------------------------------
   // A contact row is visited 13 times per substep by one thread, in color order. The row records
@@ -782,7 +790,7 @@ struct SolverT {
       }
     }
     if (ANG && (fl & PKF_ANG) != 0u) {
-      const Twists r = free_angular(row, a, b, n, t1, t2, pooled, ta0, ta1, tb0, tb1);
+      const Twists r = free_angular(*this, row, a, b, n, t1, t2, pooled, ta0, ta1, tb0, tb1);
       ta0 = r.ta0; ta1 = r.ta1; tb0 = r.tb0; tb1 = r.tb1;
     }
     if (a >= 0) { tw[2 * a] = mf4(ta0, 0.0f); tw[2 * a + 1] = mf4(ta1, 0.0f); }
@@ -858,6 +866,15 @@ struct SolverT {
         __syncthreads();
       }
     }
+    // What decides whether a row is idle, in list order: impulses and finite flag (-1: bilateral);
+    // mu, rhs, 1/K and weight.
+    for (uint32_t k = tid; k < nd; k += nt) {
+      const uint32_t row = list[k], o = S.A_DENSE + row * S.DPS;
+      const bool bil = A[o + 21u] > 0.5f;
+      S.dhd[2u * k] = make_float4(A[o + 9u], A[o + 10u], A[o + 11u], bil ? -1.0f : (S.sched[S.S_DFIN + row] != 0u ? 1.0f : 0.0f));
+      S.dhd[2u * k + 1u] = make_float4(A[o + 3u], A[o + 4u], A[o + 5u], A[o + 24u]);
+    }
+    __syncthreads();
   }
   // Dense same-articulation rows of articulation a (wgsl.js:3306-3364), one warp: lane l owns
   // dofs l, l + 32, ... (so lanes never touch each other's qd entries) and its partial sums
@@ -890,38 +907,127 @@ struct SolverT {
     d.nbil = A[o + 21u]; d.m22 = A[o + 22u]; d.m23 = A[o + 23u]; d.m24 = A[o + 24u];
     d.lam = mf3(A[o + 9u], A[o + 10u], A[o + 11u]);
   }
+  // Most of a chain's rows are contacts of links that are near but do not touch: no impulse before the
+  // visit and none after, so they change nothing. The pass looks ahead over up to 32 such rows at
+  // once: each row's normal velocity is reduced over the lanes with the additions of lane_sum (the
+  // exchange halves the rows a lane keeps at each step, so lane r ends with row r's sum), lane r
+  // decides row r, and the rows before the first that gets an impulse are done. That row, and
+  // rows that have one, go one at a time. One at a time a 40-link chain's 113 rows took 150-370
+  // thousand cycles a sweep.
+  __device__ uint32_t idle_rows(uint32_t k, uint32_t n, uint32_t it, uint32_t base0, uint32_t lane, uint32_t nw,
+                                const float (&q)[DENSE_REG], const uint32_t* dl, float4 h0) const {
+    const float* A = S.art + base0 + S.DHDR;
+    const uint32_t mine = lane < n ? dl[k + lane] : 0u;
+    const float4 h1 = lane < n ? S.dhd[2u * (k + lane) + 1u] : make_float4(0, 0, 0, 0);
+    float p[32];
+#pragma unroll
+    for (uint32_t i = 0; i < 32u; i++) {
+      const uint32_t row = __shfl_sync(0xffffffffu, mine, (int)i);
+      float s = 0.0f;
+#pragma unroll
+      for (uint32_t j = 0; j < DENSE_REG; j++) {
+        const uint32_t d = lane + 32u * j;
+        if (i < n && d < nw) s += A[(size_t)row * S.DPS + d] * q[j];
+      }
+      p[i] = s;
+    }
+#pragma unroll
+    for (uint32_t off = 16u; off > 0u; off >>= 1u) {
+      const bool up = (lane & off) != 0u;
+#pragma unroll
+      for (uint32_t i = 0; i < off; i++) {
+        const float send = up ? p[i] : p[i + off], keep = up ? p[i + off] : p[i];
+        p[i] = keep + __shfl_xor_sync(0xffffffffu, send, (int)off);
+      }
+    }
+    const float jv = p[0], w = h1.w;
+    const float nl = fmx(h0.x + S.F_OMEGA * ((((-(jv + h1.y)) * h1.z) * w) - (1.0f - w) * h0.x), 0.0f);
+    const float lim = it < S.FSTART ? 0.0f : h1.x * nl;
+    const bool idle = lane < n && __float_as_uint(nl) == 0u && lim <= 0.0f;
+    const uint32_t busy = ~__ballot_sync(0xffffffffu, idle);
+    return busy != 0u ? (uint32_t)__ffs(busy) - 1u : 32u;
+  }
   __device__ bool dense(uint32_t a, uint32_t mode, uint32_t it, uint32_t ph, uint32_t lane) const {
     const uint32_t DPS = S.DPS, base0 = S.A_DENSE;
-    const uint32_t nd = min(S.sched[S.S_META + 3u], S.MAXDENSE);
     const uint4 ai = ar.info(a);
-    if (ai.w > 32u * DENSE_REG) return dense_wide(a, mode, it, ph, lane, nd, ai);
+    uint32_t& state = S.sched[S.S_DSTATE + a];
+    if (ai.w > 32u * DENSE_REG) {
+      const bool touched = dense_wide(a, mode, it, ph, lane, min(S.sched[S.S_META + 3u], S.MAXDENSE), ai);
+      __syncwarp();
+      if (touched && lane == 0u) state &= AS_ALONE;
+      __syncwarp();
+      return touched;
+    }
     const uint32_t* dl = S.sched + S.S_DLIST;
     const uint32_t k0 = S.sched[S.S_DSTART + a], k1 = S.sched[S.S_DSTART + a + 1u];
     if (k0 >= k1) return false;
+    const uint32_t st0 = state;
+    const bool skip_twists = (st0 & (AS_ALONE | AS_FRESH)) == (AS_ALONE | AS_FRESH);
+    // The rows were all idle at this qd and nothing has moved it since: so they are again.
+    if ((st0 & AS_QUIET) != 0u && mode == 1u && ph == 0u && !vpass) return !skip_twists;
     float* qg = aqd + ai.z;
     float q[DENSE_REG];
+    bool mz = false;  // an entry -0, which adding zeros would turn into +0
 #pragma unroll
-    for (uint32_t j = 0; j < DENSE_REG; j++) q[j] = lane + 32u * j < ai.w ? qg[lane + 32u * j] : 0.0f;
-    uint32_t row = dl[k0];
-    DenseRow cur;
-    dense_load(base0 + row * DPS, lane, ai.w, cur);
-    for (uint32_t k = k0; k < k1; k++) {
-      const bool more = k + 1u < k1;
-      const uint32_t nrow = more ? dl[k + 1u] : row;
-      DenseRow nxt;
-      if (more) dense_load(base0 + nrow * DPS, lane, ai.w, nxt);
-      dense_row(cur, base0 + row * DPS, ai, mode, it, ph, lane, q);
-      cur = nxt;
-      row = nrow;
+    for (uint32_t j = 0; j < DENSE_REG; j++) {
+      q[j] = lane + 32u * j < ai.w ? qg[lane + 32u * j] : 0.0f;
+      mz = mz || __float_as_uint(q[j]) == 0x80000000u;
     }
-    (void)nd;
+    const bool ahead = !vpass && !__any_sync(0xffffffffu, mz);
+    bool moved = false;
+    uint32_t k = k0;
+    while (k < k1) {
+      if (ahead) {
+        // The run of rows from k that had no impulse; in the warm sweep they are done, and so are
+        // bilateral rows and the rows that this phase leaves out.
+        const uint32_t n = min(32u, k1 - k);
+        const float4 h0 = lane < n ? S.dhd[2u * (k + lane)] : make_float4(0, 0, 0, 0);
+        const bool bil = h0.w < 0.0f;
+        const bool left_out = ph != 0u && bil == (ph == 1u);
+        const bool zero = h0.w > 0.0f && (__float_as_uint(h0.x) | __float_as_uint(h0.y) | __float_as_uint(h0.z)) == 0u;
+        const uint32_t open = ~__ballot_sync(0xffffffffu, lane < n && (left_out || (mode == 0u ? bil || zero : zero)));
+        uint32_t run = open != 0u ? (uint32_t)__ffs(open) - 1u : 32u;
+        if (mode == 1u && ph == 0u && run > 0u) run = idle_rows(k, run, it, base0, lane, ai.w, q, dl, h0);
+        else if (mode == 1u && run > 0u) run = __shfl_sync(0xffffffffu, left_out ? 1u : 0u, 0) != 0u ? 1u : 0u;
+        if (run > 0u) {
+          k += run;
+          continue;
+        }
+      }
+      // Row k, and the rows after it that have an impulse too, one after another: the next one's
+      // data are loaded while this one is solved.
+      uint32_t row = dl[k];
+      DenseRow cur;
+      dense_load(base0 + row * DPS, lane, ai.w, cur);
+      for (;;) {
+        const bool more = k + 1u < k1;
+        const uint32_t nrow = more ? dl[k + 1u] : row;
+        const float4 nh = more ? S.dhd[2u * (k + 1u)] : make_float4(0, 0, 0, 0);
+        DenseRow nxt;
+        if (more) dense_load(base0 + nrow * DPS, lane, ai.w, nxt);
+        dense_row(cur, base0 + row * DPS, S.dhd + 2u * k, ai, mode, it, ph, lane, q);
+        moved = true;
+        k++;
+        if (!more || (ahead && nh.w > 0.0f && nh.x == 0.0f && nh.y == 0.0f && nh.z == 0.0f)) break;
+        cur = nxt;
+        row = nrow;
+      }
+    }
+    if (!moved) {
+      if (lane == 0u) state = st0 | AS_FRESH | (mode == 1u && ph == 0u && ahead ? AS_QUIET : 0u);
+      __syncwarp();
+      return !skip_twists;
+    }
 #pragma unroll
     for (uint32_t j = 0; j < DENSE_REG; j++)
       if (lane + 32u * j < ai.w) qg[lane + 32u * j] = q[j];
+    if (lane == 0u) state = (st0 & AS_ALONE) | AS_FRESH;  // the twist pass follows
+    __syncwarp();
     return true;
   }
   // One dense row (wgsl.js:3320-3362) from its registers; lane 0 stores the new impulses.
-  __device__ void dense_row(const DenseRow& d, uint32_t o, uint4 ai, uint32_t mode, uint32_t it, uint32_t ph,
+  // hd: its entry in list order, whose impulses follow.
+  __device__ void dense_row(const DenseRow& d, uint32_t o, float4* hd, uint4 ai, uint32_t mode, uint32_t it, uint32_t ph,
                             uint32_t lane, float (&q)[DENSE_REG]) const {
     float* A = S.art;
     const f3 lam = d.lam;
@@ -995,7 +1101,11 @@ struct SolverT {
       uint32_t k = lane + 32u * j;
       if (k < ai.w) q[j] += d.Y[1][j] * d1 + d.Y[2][j] * d2;
     }
-    if (lane == 0u) { A[o + 9u] = nl; A[o + 10u] = lt.x; A[o + 11u] = lt.y; }
+    if (lane == 0u) {
+      A[o + 9u] = nl; A[o + 10u] = lt.x; A[o + 11u] = lt.y;
+      hd[0] = make_float4(nl, lt.x, lt.y, hd[0].w);
+    }
+    __syncwarp();  // the look-ahead's lanes read the entry
   }
   // The same for articulations of more than 32 * DENSE_REG dofs, reading rows as it goes.
   __device__ bool dense_wide(uint32_t a, uint32_t mode, uint32_t it, uint32_t ph, uint32_t lane, uint32_t nd,
@@ -1055,11 +1165,22 @@ struct SolverT {
     }
     return touched;
   }
-  // Exact articulation update from the contact impulses on its links (wgsl.js:3380-3394).
-  __device__ void contact_impulses(uint32_t a) const {
+  // State bits of an articulation during a solve (S_DSTATE). ALONE: no contact row touches its links,
+  // so only its own joint and dense rows move it. FRESH: its link twists are those of its qd (set by a
+  // twist pass, cleared by apply). QUIET: every dense row was idle at its present qd.
+  enum : uint32_t { AS_ALONE = 1u, AS_FRESH = 2u, AS_QUIET = 4u };
+  __device__ void art_apply(uint32_t a, uint32_t lane) const {
+    __syncwarp();
+    Art::apply_warp(ar, a, aqd, tw, lane);
+    if (lane == 0u) S.sched[S.S_DSTATE + a] &= AS_ALONE;
+    __syncwarp();
+  }
+  // Exact articulation update from the contact impulses on its links (wgsl.js:3380-3394), by a warp.
+  __device__ void contact_impulses(uint32_t a, uint32_t lane) const {
+    if ((S.sched[S.S_DSTATE + a] & AS_ALONE) != 0u) return;
     uint4 ai = ar.info(a);
     bool hit = false;
-    for (uint32_t k = 0; k < ai.y; k++) {
+    for (uint32_t k = lane; k < ai.y; k += 32u) {
       uint32_t l = ai.x + k;
       uint32_t b = (uint32_t)ar.lbody(l);
       f3 f = v3(imp[b * 2u]), t = v3(imp[b * 2u + 1u]);
@@ -1070,13 +1191,25 @@ struct SolverT {
         imp[b * 2u + 1u] = make_float4(0, 0, 0, 0);
       }
     }
-    if (hit) ar.apply(a, aqd, tw);
+    if (__any_sync(0xffffffffu, hit)) art_apply(a, lane);
   }
-  // Joint friction and limit rows over the dofs listed in prepare (wgsl.js:3404-3468).
-  __device__ void joint_rows(uint32_t a) const {
+  // One joint impulse: every lane has computed it; lane 0 stores, the warp propagates it.
+  __device__ void joint_impulse(uint32_t a, uint32_t l, uint32_t r, float* slot, float value, float tau,
+                                uint32_t lane) const {
+    __syncwarp();  // every lane has read what lane 0 overwrites
+    if (lane == 0u) {
+      if (slot != nullptr) *slot = value;
+      ar.LB[ar.lo(l) + L_TAU + r] = tau;
+    }
+    art_apply(a, lane);
+  }
+  // Joint friction and limit rows over the dofs listed in prepare (wgsl.js:3404-3468), by a warp: the
+  // lanes compute each row alike (one after another, as each moves qd) and share its propagation.
+  __device__ void joint_rows(uint32_t a, uint32_t lane) const {
     float* A = S.art;
-    uint4 ai = ar.info(a);
     uint32_t n = f2u(A[S.A_RLN + a]);
+    if (n == 0u) return;
+    uint4 ai = ar.info(a);
     for (uint32_t i = 0; i < n; i++) {
       uint32_t d = f2u(A[S.A_RL + ai.z + i]);
       uint32_t l = f2u(ar.dof_limit(d).w);
@@ -1095,14 +1228,14 @@ struct SolverT {
         float mx = dr.w > 0.0f ? dr.w * P.dt : 1e20f;
         float lam = A[S.A_DRV + d];
         float nl = clmp((lam * (1.0f - x) - (x * ca) * aqd[d]) + bias, -mx, mx);
-        if (nl != lam) { A[S.A_DRV + d] = nl; ar.LB[ar.lo(l) + L_TAU + r] = nl - lam; ar.apply(a, aqd, tw); }
+        if (nl != lam) joint_impulse(a, l, r, &A[S.A_DRV + d], nl, nl - lam, lane);
       }
       float fr = ar.dof_passive(d).y;
       if (S.JFL == 1u) fr += A[S.A_JFL + d];
       if (fr > 0.0f) {
         float lam = A[S.A_FRIC + d];
         float nl = clmp(lam - (S.F_OMEGA * aqd[d]) / hinv, -fr * P.dt, fr * P.dt);
-        if (nl != lam) { A[S.A_FRIC + d] = nl; ar.LB[ar.lo(l) + L_TAU + r] = nl - lam; ar.apply(a, aqd, tw); }
+        if (nl != lam) joint_impulse(a, l, r, &A[S.A_FRIC + d], nl, nl - lam, lane);
       }
       float4 lim = ar.dof_limit(d);
       if (A[S.A_LG + d] > 0.5f) {
@@ -1115,16 +1248,14 @@ struct SolverT {
           if (gap < 0.0f) rhs = vpass ? 0.0f : fmx((P.beta * gap) / P.dt, -P.max_depen);
           float nl = fmx(lam - (S.F_OMEGA * (sg * aqd[d] + rhs)) / hinv, 0.0f);
           if (nl == lam) continue;
-          A[S.A_LIM + 2u * d + side] = nl;
-          ar.LB[ar.lo(l) + L_TAU + r] = sg * (nl - lam);
-          ar.apply(a, aqd, tw);
+          joint_impulse(a, l, r, &A[S.A_LIM + 2u * d + side], nl, sg * (nl - lam), lane);
         }
       }
     }
   }
   // Joint velocity limits after the contact impulses (wgsl.js:3413-3419, 3462-3467): a stateless
-  // push back onto |qd| <= limit for the marked dofs of revolute, prismatic and D6 links.
-  __device__ void vlim_rows(uint32_t a) const {
+  // push back onto |qd| <= limit for the marked dofs of revolute, prismatic and D6 links. By a warp.
+  __device__ void vlim_rows(uint32_t a, uint32_t lane) const {
     float* A = S.art;
     if (A[S.A_AVL + a] <= 0.5f) return;
     uint4 ai = ar.info(a);
@@ -1137,7 +1268,7 @@ struct SolverT {
         float4 pv = ar.dof_passive(d);
         if (pv.z >= 0.0f && A[S.A_VLG + d] > 0.5f) {
           float over = aqd[d] - clmp(aqd[d], -pv.z, pv.z);
-          if (over != 0.0f) { ar.LB[ar.lo(l) + L_TAU + r] = (-over) / hinv; ar.apply(a, aqd, tw); }
+          if (over != 0.0f) joint_impulse(a, l, r, nullptr, 0.0f, (-over) / hinv, lane);
         }
       }
     }
@@ -1262,9 +1393,9 @@ struct SolverT {
         momentum_unit(S.sched[S.S_RUNIT + row], row, beta, it == 0u);
       }
     __syncthreads();
-    for (uint32_t a = tid; a < S.NA; a += nt) {
-      contact_impulses(a);
-      if (S.VLIM_ON == 1u) vlim_rows(a);
+    for (uint32_t a = tid >> 5u; a < S.NA; a += nt >> 5u) {
+      contact_impulses(a, tid & 31u);
+      if (S.VLIM_ON == 1u) vlim_rows(a, tid & 31u);
     }
     __syncthreads();
   }
@@ -1278,8 +1409,9 @@ struct SolverT {
     const uint32_t tid = tm.rank(), nt = tm.size();
     const uint32_t ncol = ph == 2u ? 0u : ncol0;
     const bool pk_on = packed();
+    const uint32_t lane = threadIdx.x & 31u;  // a warp per articulation
     if (ph != 1u)
-      for (uint32_t a = tid; a < S.NA; a += nt) joint_rows(a);
+      for (uint32_t a = tid >> 5u; a < S.NA; a += nt >> 5u) joint_rows(a, lane);
     if (S.PATCH == 1u && mode == 1u) {
       // Four units per thread at a time, their loads issued together (each unit's sum keeps its
       // row order).
@@ -1325,9 +1457,9 @@ struct SolverT {
         for (uint32_t u = wcs[S.NCOL]; u < wcs[S.NCOL + 1u]; u++) solve_slot<EXT>(u, mode, it);
     }
     tm.sync();
-    for (uint32_t a = tid; a < S.NA; a += nt) {
-      contact_impulses(a);
-      if (S.VLIM_ON == 1u && ph != 1u) vlim_rows(a);
+    for (uint32_t a = tid >> 5u; a < S.NA; a += nt >> 5u) {
+      contact_impulses(a, lane);
+      if (S.VLIM_ON == 1u && ph != 1u) vlim_rows(a, lane);
     }
     tm.sync();
     if (S.VLIM_FREE == 1u) {
@@ -1477,6 +1609,13 @@ __device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team
       const size_t o = SolverT<TEAM>::pk_offset(wcs, c, u - wcs[c]);
       sv.pack_row((rows_shared && !TEAM && c < ncol ? rows_sm : pk_global) + o, row, us, key);
     }
+  }
+  // An articulation no contact row touches: prepare marked the bodies of the others' links.
+  for (uint32_t a = tid; a < S.NA; a += nt) {
+    const uint4 ai = sv.ar.info(a);
+    bool alone = true;
+    for (uint32_t k = 0; k < ai.y; k++) alone = alone && S.sched[S.S_LINKHIT + (uint32_t)sv.ar.lbody(ai.x + k)] == 0u;
+    S.sched[S.S_DSTATE + a] = SolverT<TEAM>::AS_FRESH | (alone ? SolverT<TEAM>::AS_ALONE : 0u);
   }
   tm.sync();
   // Few articulations: a warp each (the chain recursion shortened); many: a thread each.

@@ -1,0 +1,79 @@
+"""The solve's packed contact rows and its look-ahead over idle dense rows, bit for bit against the
+oracle at the sizes where they can go wrong: colors with a partly filled tile, rows in shared and in
+global memory, chains around the lane count and the register-held dofs, with contacts between their
+links that push and contacts that do not."""
+import math
+
+import numpy as np
+import pytest
+
+from steel_webgpu_b200 import SceneBuilder, pack, synth
+from steel_webgpu_b200.sim import Batch
+
+pytestmark = pytest.mark.gpu
+
+# Room for every pair of the dense scenes below (what a full buffer drops depends on the order).
+ROOM = 16384
+CAPS = dict(MAXP=ROOM, MAXC=ROOM, MAXU=ROOM, UH=ROOM, WH=2 * ROOM, AH=ROOM, MAXDENSE=ROOM)
+
+
+def _bits(a):
+    return np.ascontiguousarray(a).view(np.uint32)
+
+
+def _same_as_oracle(pk, oracle_lib, frames, tiles=()):
+    o = oracle_lib.OracleSim(pk)
+    g = Batch([pk])
+    if tiles:
+        g.set_tiles(*tiles)
+    for _ in range(2):
+        o.step(frames)
+        g.step(frames)
+        assert not g.stats()["overflow"]
+        pose, vel, q, qd, _ = g.raw_state()
+        art = o.read("art")
+        assert np.array_equal(_bits(o.read("poses")[:pk.NB * 8]), _bits(pose))
+        assert np.array_equal(_bits(o.read("vel")[:pk.NB * 8]), _bits(vel))
+        assert np.array_equal(_bits(art[pk.C["A_Q"]:pk.C["A_Q"] + pk.NQ]), _bits(q))
+        assert np.array_equal(_bits(art[pk.C["A_QD"]:pk.C["A_QD"] + pk.ND]), _bits(qd))
+    stats = g.stats()
+    g.close()
+    return stats
+
+
+def _chains(links, fold):
+    """Two chains, one hanging straight, one folded by `fold` rad a joint onto itself."""
+    b = SceneBuilder(fps=240)
+    b.add_ground_plane(mu=0.6)
+    for x, bend in ((0.0, 0.0), (2.0, fold)):
+        parent, at = -1, [x, 0.0, 8.0]
+        for k in range(links):
+            body = b.add_body(xform=[x, 0.0, 8.0 - 0.1 * (k + 0.5), 0, 0, 0, 1])
+            b.add_shape_capsule(body, radius=0.02, half_height=0.04, mass=0.2 + 0.05 * (k % 3))
+            b.add_joint_revolute(parent, body, axis=[0, 1, 0], parent_xform=at + [0, 0, 0, 1],
+                                 child_xform=[0, 0, 0.05, 0, 0, 0, 1], q=[bend], targetKe=2.0, targetKd=0.05)
+            parent, at = body, [0.0, 0.0, -0.05]
+    return b.finalize()
+
+
+@pytest.mark.parametrize("links", [2, 3, 31, 32, 33, 64, 65])
+def test_dense_rows(links, steel, oracle_lib):
+    scene = _chains(links, 2.0)  # links two apart overlap at 2 rad a joint
+    stats = _same_as_oracle(pack(scene, caps=CAPS), oracle_lib, 4)
+    assert links < 3 or stats["max_dense"] > 0
+
+
+@pytest.mark.parametrize("boxes", [1, 2, 7, 9, 33, 100])
+@pytest.mark.parametrize("tiles", [(), (512, 4096), (32, 4096)])
+def test_packed_rows(boxes, tiles, steel, oracle_lib):
+    rng = np.random.default_rng(boxes)
+    b = SceneBuilder(fps=240, box_hulls="direct")
+    b.add_ground_plane(mu=0.6)
+    side = max(1, int(math.sqrt(boxes / 3)))
+    for i in range(boxes):
+        layer, cell = divmod(i, side * side)
+        body = b.add_body(xform=[0.21 * (cell % side), 0.21 * (cell // side), 0.101 + 0.2 * layer] + synth._rand_quat(rng)
+                          if i % 5 == 4 else [0.21 * (cell % side), 0.21 * (cell // side), 0.101 + 0.2 * layer, 0, 0, 0, 1])
+        b.add_shape_box(body, hx=0.1, hy=0.1, hz=0.1, mu=0.6)
+    scene = b.finalize()
+    _same_as_oracle(pack(scene, caps=CAPS), oracle_lib, 15, tiles)
