@@ -549,6 +549,271 @@ struct Art {
     }
   }
 
+  // --- the factorisation by one warp (all 32 lanes call it) -----------------------------------
+  // One thread took 4,000-9,000 cycles a link (40 links: 180 us of a 128-thread block's prepare, 780
+  // us with eight blocks on the SM). Here the velocities go down the tree by level; bias forces and
+  // link inertias are a lane per link; the inertia's way to the root takes the links in the serial
+  // order with a lane per matrix element (backward_link); the accelerations go down by level. Every
+  // element is computed by the serial pass's operations in its order.
+  template <class T> static __device__ __forceinline__ T lane_get(T v, uint32_t src) {
+    return __shfl_sync(0xffffffffu, v, (int)src);
+  }
+  // Component j of I^A m for the inertia at o, read as floats (imul, one component).
+  template <class T>
+  __device__ T imul_comp(uint32_t o, uint32_t j, T ax, T ay, T az, T lx, T ly, T lz) const {
+    const uint32_t i = j < 3u ? j : j - 3u;
+    const uint32_t b0 = o + (j < 3u ? i : 9u + 3u * i), s0 = j < 3u ? 3u : 1u, b1 = o + (j < 3u ? 9u : 18u) + i;
+    return (((T)LB[b0] * ax + (T)LB[b0 + s0] * ay) + (T)LB[b0 + 2u * s0] * az) +
+           (((T)LB[b1] * lx + (T)LB[b1 + 3u] * ly) + (T)LB[b1 + 6u] * lz);
+  }
+  // Backward step of link l. T: float, or double for ART_F64, whose inertia, U, D and its inverse and
+  // the parent's sum are computed in double from the stored floats and rounded on store (back_f64).
+  // Lane e < 27 owns element e of (A, B, C), lane j < 6 component j of U and of the bias force, lane
+  // c < 6 column c of D, lane 8 + c column c of its inverse.
+  template <class T>
+  __device__ void backward_link(uint32_t l, const Params& P, uint32_t lane) const {
+    const uint32_t JM = JMc, L = lo(l), n = lndof(l), d0 = ldof(l), qs = lqs(l);
+    const int par = lparent(l);
+    const uint32_t em = lane / 9u, ec = (lane % 9u) / 3u, ei = lane % 3u, j6 = lane < 6u ? lane : 0u;
+    T el = lane < 27u ? (T)LB[L + L_IA + lane] : (T)0;
+    const SVec pA = ldsv(L + L_PA);
+    T uj[6];  // component `lane` of U_c
+#pragma unroll
+    for (uint32_t c = 0; c < 6u; c++) {
+      uj[c] = (T)0;
+      if (c < n) {
+        const SVec s = ldS(l, c);
+        uj[c] = imul_comp<T>(L + L_IA, j6, (T)s.a.x, (T)s.a.y, (T)s.a.z, (T)s.l.x, (T)s.l.y, (T)s.l.z);
+        if (lane < 6u) LB[L + L_U + c * 6u + lane] = (float)uj[c];
+      }
+    }
+    // Column c of D = S^T U on lane c, with the drive and damping terms on the diagonal.
+    T uc[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (uint32_t c = 0; c < 6u; c++) {
+      if (c >= n) break;
+#pragma unroll
+      for (uint32_t j = 0; j < 6u; j++) {
+        const T v = lane_get(uj[c], j);
+        if (lane == c) uc[j] = v;
+      }
+    }
+    T v[6] = {0, 0, 0, 0, 0, 0};  // rows of this lane's column of D (lanes < 6) or of the inverse (8 + c)
+    float u = 0.0f;
+    if (lane < n) {
+      T diag = (T)0;
+#pragma unroll
+      for (uint32_t r = 0; r < 6u; r++) {
+        if (r >= n) break;
+        const SVec s = ldS(l, r);
+        v[r] = (((T)s.a.x * uc[0] + (T)s.a.y * uc[1]) + (T)s.a.z * uc[2]) +
+               (((T)s.l.x * uc[3] + (T)s.l.y * uc[4]) + (T)s.l.z * uc[5]);
+        if (r == lane) diag = v[r];
+      }
+      const float tau = dof_tau(d0 + lane, qs, lane, diag, P);
+      u = tau - sdot(ldS(l, lane), pA);
+#pragma unroll
+      for (uint32_t r = 0; r < 6u; r++) if (r == lane) v[r] = diag;
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < 6u; r++) if (lane == 8u + r) v[r] = (T)1;
+    // Gauss-Jordan inverse (inv_spd), a column per lane.
+#pragma unroll
+    for (uint32_t c = 0; c < 6u; c++) {
+      if (c >= n) break;
+      const T piv = lane_get(v[c], c);
+      const T least = (T)1e-12, pv = (T)1 / (least > piv ? least : piv);
+      v[c] *= pv;
+#pragma unroll
+      for (uint32_t r = 0; r < 6u; r++) {
+        if (r >= n) break;
+        if (r == c) continue;
+        const T f = lane_get(v[r], c);
+        if (f != (T)0) v[r] -= f * v[c];
+      }
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < 6u; r++) {
+      if (r >= JM) break;
+      if (lane >= 8u && lane < 8u + JM) LB[L + L_DI + r * JM + (lane - 8u)] = r < n && lane - 8u < n ? (float)v[r] : 0.0f;
+    }
+    if (lane < JM) LB[L + L_UU + lane] = lane < n ? u : 0.0f;
+    if (par < 0) {
+      __syncwarp();
+      return;
+    }
+    // Projection: I^A - U D^-1 U^T, element by element over (r, c); and U D^-1 u.
+    T x[6], y[6];
+#pragma unroll
+    for (uint32_t c = 0; c < 6u; c++) {
+      x[c] = y[c] = (T)0;
+      if (c >= n) break;
+      x[c] = lane_get(uj[c], (em == 2u ? 3u : 0u) + ei);
+      y[c] = lane_get(uj[c], (em == 0u ? 0u : 3u) + ec);
+    }
+    float duu = 0.0f;
+#pragma unroll
+    for (uint32_t r = 0; r < 6u; r++) {
+      if (r >= n) break;
+      float du = 0.0f;
+#pragma unroll
+      for (uint32_t c = 0; c < 6u; c++) {
+        if (c >= n) break;
+        const T w = lane_get(v[r], 8u + c);
+        el -= w * (x[r] * y[c]);
+        du += (float)w * lane_get(u, c);
+      }
+      duu += (float)uj[r] * du;
+    }
+    __syncwarp();  // every lane has read the inertia
+    if (lane < 27u) LB[L + L_IA + lane] = (float)el;
+    __syncwarp();
+    const SVec cb = ldsv(L + L_C);
+    const float pa0 = j6 < 3u ? comp(pA.a, (int)j6) : comp(pA.l, (int)j6 - 3);
+    const float pa = (pa0 + imul_comp<float>(L + L_IA, j6, cb.a.x, cb.a.y, cb.a.z, cb.l.x, cb.l.y, cb.l.z)) + duu;
+    // Into the parent, shifted by r: A' = A + Am - Bm Rs + Rs Bm^T - Rs Cm Rs, B' = B + Bm + Rs Cm,
+    // C' = C + Cm. Rs[c][i] is component i of column c.
+    const uint32_t P0 = lo((uint32_t)par);
+    const f3 rf = link_r(l);
+    const T rx = (T)rf.x, ry = (T)rf.y, rz = (T)rf.z;
+    auto rs = [&](uint32_t c, uint32_t i) -> T {
+      if (c == i) return (T)0;
+      if (c == 0u) return i == 1u ? rz : -ry;
+      if (c == 1u) return i == 0u ? -rz : rx;
+      return i == 0u ? ry : -rx;
+    };
+    // Rs Cm, element (ec, ei), on every lane.
+    const T t = (rs(0u, ei) * lane_get(el, 18u + 3u * ec) + rs(1u, ei) * lane_get(el, 19u + 3u * ec)) +
+                rs(2u, ei) * lane_get(el, 20u + 3u * ec);
+    const T br = (lane_get(el, 9u + ei) * rs(ec, 0u) + lane_get(el, 12u + ei) * rs(ec, 1u)) + lane_get(el, 15u + ei) * rs(ec, 2u);
+    const T rb = (rs(0u, ei) * lane_get(el, 9u + ec) + rs(1u, ei) * lane_get(el, 12u + ec)) + rs(2u, ei) * lane_get(el, 15u + ec);
+    const T tr_ = (lane_get(t, ei) * rs(ec, 0u) + lane_get(t, 3u + ei) * rs(ec, 1u)) + lane_get(t, 6u + ei) * rs(ec, 2u);
+    const T pe = lane < 27u ? (T)LB[P0 + L_IA + lane] : (T)0;
+    T sum = pe + el;
+    if (em == 0u) sum = ((sum - br) + rb) - tr_;
+    else if (em == 1u) sum = sum + t;
+    const float fx = lane_get(pa, 3u), fy = lane_get(pa, 4u), fz = lane_get(pa, 5u);
+    const f3 cr = cross(rf, mf3(fx, fy, fz));
+    const float sh = j6 < 3u ? pa + comp(cr, (int)j6) : pa;
+    if (lane < 27u) LB[P0 + L_IA + lane] = (float)sum;
+    if (lane < 6u) LB[P0 + L_PA + lane] = LB[P0 + L_PA + lane] + sh;
+    __syncwarp();
+  }
+  // Velocity of link l from its parent's (the part of factor's first pass that goes down the tree).
+  __device__ void link_velocity(uint32_t l, SVec& vp, SVec& sq) const {
+    const int par = lparent(l);
+    const uint32_t nd = lndof(l), d0 = ldof(l);
+    vp = sv0();
+    if (par >= 0) vp = mshift(ldsv(lo((uint32_t)par) + L_V), link_r(l));
+    sq = sv0();
+#pragma unroll
+    for (uint32_t c = 0; c < 6u; c++) {
+      if (c >= nd) break;
+      sq = sadd(sq, sscl(ldS(l, c), A[S.A_QD + d0 + c]));
+    }
+  }
+  template <bool F64>
+  __device__ void factor_warp(uint32_t a, const Params& P, uint32_t lane) const {
+    const uint4 ai = info(a);
+    const f3 g = v3(P.gravity);
+    const uint32_t r0 = S.lt[a], r1 = S.lt[a + 1u];
+    RO<uint32_t> lvo = S.lt + S.LT_LVO, lvl = S.lt + S.LT_LVL;
+    for (uint32_t k = r0; k < r1; k++) {
+      const uint32_t e = lvo[k + 1u];
+      for (uint32_t i = lvo[k] + lane; i < e; i += 32u) {
+        SVec vp, sq;
+        link_velocity(lvl[i], vp, sq);
+        stsv(lo(lvl[i]) + L_V, sadd(vp, sq));
+      }
+      __syncwarp();
+    }
+    for (uint32_t k = lane; k < ai.y; k += 32u) link_bias(ai.x + k, g);
+    __syncwarp();
+    for (uint32_t k = ai.y; k-- > 0u;) {
+      if (F64) backward_link<double>(ai.x + k, P, lane);
+      else backward_link<float>(ai.x + k, P, lane);
+    }
+    for (uint32_t k = r0; k < r1; k++) {
+      const uint32_t e = lvo[k + 1u];
+      for (uint32_t i = lvo[k] + lane; i < e; i += 32u) link_accel(lvl[i], g, P);
+      __syncwarp();
+    }
+  }
+  // Bias force, velocity-product acceleration and inertia of link l at its velocity L_V.
+  __device__ void link_bias(uint32_t l, f3 g) const {
+    const uint32_t L = lo(l), nd = lndof(l), d0 = ldof(l);
+    const uint32_t bo = S.A_BF + (uint32_t)lbody(l) * 8u;
+    const f3 bforce = ald3(bo), btorque = ald3(bo + 4u);
+    SVec vp, sq;
+    link_velocity(l, vp, sq);
+    const SVec v = ldsv(L + L_V);
+    SVec cb = crm(vp, sq);
+    uint32_t jt = ltype(l);
+    if (jt == 6u) {
+      uint32_t nlin = f2u(lrec(l, 5).w);
+      f3 ca = sp3(0.0f);
+      for (uint32_t j = nlin; j < nd; j++)
+        for (uint32_t kk = j + 1u; kk < nd; kk++)
+          ca += (cross(ldS(l, j).a, ldS(l, kk).a) * A[S.A_QD + d0 + j]) * A[S.A_QD + d0 + kk];
+      cb = sadd(cb, SVec{ca, cross(ca, ld3(L + L_JR))});
+    }
+    if (jt == 4u || jt == 6u) {
+      uint32_t nlin = jt == 4u ? 3u : f2u(lrec(l, 5).w);
+      f3 vo = sp3(0.0f), wj = sp3(0.0f);
+      for (uint32_t c = 0; c < nd; c++) {
+        SVec sc = ldS(l, c);
+        float q = A[S.A_QD + d0 + c];
+        if (c < nlin) vo += sc.l * q; else wj += sc.a * q;
+      }
+      cb = sadd(cb, SVec{sp3(0.0f), -cross(wj, vo)});
+    }
+    stsv(L + L_C, cb);
+    int b = lbody(l);
+    float m = bmass(b);
+    m3 R = qmat(link_rot(l));
+    m3 Ic = mul(mul(R, binertia(b)), tr(R));
+    stm(L + L_IA, Ic);
+    stm(L + L_IA + 9u, mcols(sp3(0), sp3(0), sp3(0)));
+    stm(L + L_IA + 18u, mcols(mf3(m, 0, 0), mf3(0, m, 0), mf3(0, 0, m)));
+    SVec pa0 = crf(v, imul(L + L_IA, v));
+    if ((f2u(BR[(uint32_t)b * 8u + 7u].w) & 2u) != 0u) pa0 = sadd(pa0, SVec{sp3(0.0f), m * g});
+    pa0 = sadd(pa0, SVec{-btorque, -bforce});
+    stsv(L + L_PA, pa0);
+  }
+  // Acceleration of link l from its parent's, and its free joint velocities.
+  __device__ void link_accel(uint32_t l, f3 g, const Params& P) const {
+    const uint32_t L = lo(l);
+    int par = lparent(l);
+    SVec ap = SVec{sp3(0.0f), -g};
+    if (par >= 0) ap = mshift(ldsv(lo((uint32_t)par) + L_A), link_r(l));
+    const SVec a1 = sadd(ap, ldsv(L + L_C));
+    const uint32_t n = lndof(l), d0 = ldof(l);
+    SVec acc = a1;
+    float ua[6];  // U_c . a1, the same for every row
+#pragma unroll
+    for (uint32_t c = 0; c < 6u; c++) ua[c] = c < n ? LB[L + L_UU + c] - sdot(ldU(l, c), a1) : 0.0f;
+#pragma unroll
+    for (uint32_t r = 0; r < 6u; r++) {
+      if (r >= n) break;
+      float qdd = 0.0f;
+#pragma unroll
+      for (uint32_t c = 0; c < 6u; c++) {
+        if (c >= n) break;
+        qdd += ldDI(l, r, c) * ua[c];
+      }
+      A[S.A_QDH + d0 + r] = A[S.A_QD + d0 + r] + P.dt * qdd;
+      acc = sadd(acc, sscl(ldS(l, r), qdd));
+    }
+    stsv(L + L_A, acc);
+    if (S.JFL == 1u) {
+      // joint_friction_load_coefficient (artwgsl.js:361-367): the joint's transmitted force and
+      // torque under the free dynamics (I^A a + p^A at the child COM) raise its friction bound.
+      const SVec f = sadd(imul(L + L_IA, acc), ldsv(L + L_PA));
+      const float fm = len(f.l) + len(f.a);
+      for (uint32_t r = 0; r < n; r++) A[S.A_JFL + d0 + r] = DR[(d0 + r) * 5u + 3u].w * fm;
+    }
+  }
+
   __device__ uint32_t path(uint32_t l0, uint32_t* pth) const {
     uint32_t n = 0;
     int l = (int)l0;

@@ -33,6 +33,10 @@ static __constant__ float BP_BZ[20] = {0.33333337f, 0.74535593f, 0.33333330f, -0
                                 -0.74535609f, 0.74535599f, 0.33333335f, 0.74535603f, 1.0f, -0.33333335f,
                                 0.33333337f, -1.0f, -0.74535609f, 0.33333339f, 0.33333340f, -0.33333334f,
                                 -0.74535597f, -0.33333332f};
+// fcos and fsin of (float)k * 1.0471975511965976f, the six directions of a contact group's extremes
+// (39 evaluations of the double-precision series per contact and substep took 15% of the prepare).
+static __constant__ float BP_COS[6] = {0x1.0000000000000p+0f, 0x1.fffffe0000000p-2f, -0x1.0000020000000p-1f, -0x1.0000000000000p+0f, -0x1.fffffa0000000p-2f, 0x1.fffffa0000000p-2f};
+static __constant__ float BP_SIN[6] = {0.0f, 0x1.bb67b00000000p-1f, 0x1.bb67ae0000000p-1f, -0x1.777a5c0000000p-24f, -0x1.bb67b00000000p-1f, -0x1.bb67b00000000p-1f};
 static constexpr uint32_t AVN = 14u;
 
 struct Prep {
@@ -163,8 +167,8 @@ struct Prep {
   static __device__ void bp_value(float px, float py, float gap, uint32_t pk, uint32_t q, uint32_t* sc_, uint32_t* id) {
     if (q == 6u) { *sc_ = fflip(-gap); *id = pk; return; }
     if (q > 6u && gap > 0.0f) { *sc_ = 0u; *id = 0u; return; }
-    float ang = (float)(q > 6u ? q - 7u : q) * 1.0471975511965976f;
-    *sc_ = fflip(dot(mf2(px, py), mf2(fcos(ang), fsin(ang))));
+    const uint32_t k = q > 6u ? q - 7u : q;
+    *sc_ = fflip(dot(mf2(px, py), mf2(BP_COS[k], BP_SIN[k])));
     *id = pk;
   }
   static __device__ uint32_t anchor_hash(uint32_t pair, uint32_t k) { return max(mix32(pair * 2u + k), 1u); }
@@ -832,7 +836,8 @@ __device__ __forceinline__ void prepare_scene(const BatchDev& B, uint32_t sc, Te
   }
   tm.sync();
   // Joint-limit gating, listed joint rows, FK and factorisation per articulation.
-  auto gate = [&](uint32_t a) {
+  // One articulation's gating by the threads lane, lane + step, ... (a warp, or one thread: 0, 1).
+  auto gate = [&](uint32_t a, uint32_t lane, uint32_t step) {
     uint4 ai = ar.info(a);
     // Joint velocity limits (wgsl.js:1829-1854): scale the articulation's scalar dof speeds so the
     // most exceeded limit is met, then mark the dofs near their limit (rows exist only there).
@@ -841,7 +846,7 @@ __device__ __forceinline__ void prepare_scene(const BatchDev& B, uint32_t sc, Te
       const float4 dr = ar.dof_drive(d);
       return S.DRIVE_ROWS == 1u && S.FUSE_VLIM == 1u && (dr.y > 0.0f || dr.z > 0.0f);
     };
-    if (S.VLIM_ON == 1u) {
+    if (S.VLIM_ON == 1u && lane == 0u) {
       float ratio = 1.0f;
       for (uint32_t k = 0; k < ai.w; k++) {
         uint32_t d = ai.z + k;
@@ -862,42 +867,51 @@ __device__ __forceinline__ void prepare_scene(const BatchDev& B, uint32_t sc, Te
       }
       A[S.A_AVL + a] = any ? 1.0f : 0.0f;
     }
+    if (step > 1u) __syncwarp();  // the scaled speeds
     uint32_t n = 0u;
-    for (uint32_t k = 0; k < ai.w; k++) {
-      uint32_t d = ai.z + k;
-      float4 lim = ar.dof_limit(d);
-      bool on = false;
-      if (lim.z > 0.5f) {
-        uint32_t l = f2u(lim.w);
-        float q = A[S.A_Q + ar.lqs(l) + d - ar.ldof(l)];
-        float g = S.F_JL_GAP + (S.F_JL_SPEED * P.dt) * fabsf(A[S.A_QD + d]);
-        on = q <= lim.x + g || q >= lim.y - g;
+    for (uint32_t k0 = 0; k0 < ai.w; k0 += step) {
+      const uint32_t k = k0 + lane, d = ai.z + k;
+      bool row = false;
+      if (k < ai.w) {
+        float4 lim = ar.dof_limit(d);
+        bool on = false;
+        if (lim.z > 0.5f) {
+          uint32_t l = f2u(lim.w);
+          float q = A[S.A_Q + ar.lqs(l) + d - ar.ldof(l)];
+          float g = S.F_JL_GAP + (S.F_JL_SPEED * P.dt) * fabsf(A[S.A_QD + d]);
+          on = q <= lim.x + g || q >= lim.y - g;
+        }
+        A[S.A_LG + d] = on ? 1.0f : 0.0f;
+        const float4 drv = ar.dof_drive(d);
+        row = (on || ar.dof_passive(d).y > 0.0f || S.JFL == 1u || (S.DRIVE_ROWS == 1u && (drv.y > 0.0f || drv.z > 0.0f))) &&
+              ar.scalar_dof(d);
       }
-      A[S.A_LG + d] = on ? 1.0f : 0.0f;
-      const float4 drv = ar.dof_drive(d);
-      bool row = on || ar.dof_passive(d).y > 0.0f || S.JFL == 1u || (S.DRIVE_ROWS == 1u && (drv.y > 0.0f || drv.z > 0.0f));
-      if (row && ar.scalar_dof(d)) { A[S.A_RL + ai.z + n] = (float)d; n++; }
+      // Listed in dof order.
+      const uint32_t rows = step > 1u ? __ballot_sync(0xffffffffu, row) : (row ? 1u : 0u);
+      if (row) A[S.A_RL + ai.z + n + (uint32_t)__popc(rows & ((1u << lane) - 1u))] = (float)d;
+      n += (uint32_t)__popc(rows);
     }
-    A[S.A_RLN + a] = (float)n;
+    if (lane == 0u) A[S.A_RLN + a] = (float)n;
   };
   auto factor = [&](uint32_t a) {
     if (F64 && S.ART_F64 == 1u) ar.factor<true>(a, P);
     else ar.factor<false>(a, P);
   };
-  if (S.NA <= (nt >> 5u)) {
-    // Few articulations: a warp each, so the FK's per-link trigonometry and outputs run across
-    // lanes and only the pose chain is serial.
+  if (S.NA <= 4u * (nt >> 5u)) {
+    // Few articulations: a warp each, lanes over links and matrix elements. Beyond four to a warp a
+    // thread each has more of them in flight.
     const uint32_t lane = tid & 31u;
     for (uint32_t a = tid >> 5u; a < S.NA; a += nt >> 5u) {
-      if (lane == 0u) gate(a);
+      gate(a, lane, 32u);
       __syncwarp();
       ar.fk_warp(a, lane);
-      if (lane == 0u) factor(a);
+      if (F64 && S.ART_F64 == 1u) ar.template factor_warp<true>(a, P, lane);
+      else ar.template factor_warp<false>(a, P, lane);
       __syncwarp();
     }
   } else {
     for (uint32_t a = tid; a < S.NA; a += nt) {
-      gate(a);
+      gate(a, 0u, 1u);
       ar.fk(a);
       factor(a);
     }
