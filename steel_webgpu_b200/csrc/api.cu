@@ -89,7 +89,7 @@ struct SceneHost {
   SceneDev d{};  // device pointers filled after allocation
   // arena offsets
   size_t o_sf, o_su, o_pos, o_rot, o_ppos, o_prot, o_lv, o_av, o_spos, o_srot, o_alo, o_ahi, o_art, o_cnt, o_stats,
-      o_params, o_craw, o_con, o_ckeys, o_rows, o_slots, o_pk, o_plam, o_warm, o_sched, o_tw, o_imp, o_aqd, o_tscr;
+      o_params, o_craw, o_con, o_ckeys, o_rows, o_slots, o_pk, o_plam, o_bpc, o_warm, o_sched, o_tw, o_imp, o_aqd, o_tscr;
   // Device-wide radix sort of a scene whose padded keys may exceed the block sort's shared array.
   bool large_sort = false;
   uint32_t sort_tiles = 0;
@@ -283,8 +283,8 @@ int build_scene(SceneHost& s, const steel_scene_desc& in, Layout& L, uint32_t th
     auto put = [&](uint32_t& field, size_t n) { field = (uint32_t)so; so += n > 0 ? n : 1; };
     put(d.S_UNITOF, MAXC); put(d.S_DSLOT, MAXC); put(d.S_CORDER, MAXC); put(d.S_UKEY, MAXC);
     put(d.S_USTART0, MAXC + 1); put(d.S_USIZE, MAXC); put(d.S_USTART, MAXC + 1); put(d.S_RK0, MAXC);
-    put(d.S_RK1, MAXC); put(d.S_RK2, MAXC); put(d.S_BPC, 4 * (size_t)MAXC); put(d.S_LEAD, MAXC);
-    put(d.S_KEEP, MAXC); put(d.S_SLOT, 26 * (size_t)MAXC); put(d.S_KEPT, MAXC); put(d.S_ROWOF, MAXC);
+    put(d.S_RK1, MAXC); put(d.S_RK2, MAXC); put(d.S_LEAD, MAXC);
+    put(d.S_KEEP, MAXC); put(d.S_KEPT, MAXC); put(d.S_ROWOF, MAXC);
     put(d.S_RUNIT, MAXC); put(d.S_RCON, MAXC); put(d.S_PCOL, MAXC); put(d.S_PORD, MAXC);
     put(d.S_CSTART, d.NCOL + 2); put(d.S_META, 8); put(d.S_WWIN, d.WH); put(d.S_WSLOT, (size_t)MAXC + d.MAXDENSE);
     put(d.S_WMASK, (size_t)NB * d.NCOLW); put(d.S_WCOUNT, d.NCOL + 2); put(d.S_LINKHIT, NB); put(d.S_JSPLIT, NL);
@@ -349,6 +349,7 @@ int build_scene(SceneHost& s, const steel_scene_desc& in, Layout& L, uint32_t th
   }
   s.o_rows = L.take((size_t)MAXC * d.ROWS * 16); s.o_slots = L.take((size_t)MAXC * 2 * 16);
   s.o_pk = L.take(((size_t)MAXC / 8u + d.NCOL + 8u) * PK_TILE); s.o_plam = L.take((size_t)MAXC * 4);
+  s.o_bpc = L.take((size_t)MAXC * 16);
   s.o_warm = L.take(s.warm_words * 4);
   s.o_sched = L.take(s.sched_words * 4);
   s.o_tw = L.take((size_t)NB * 32); s.o_imp = L.take((size_t)NB * 32);
@@ -793,6 +794,7 @@ int steel_batch_create(steel_ctx* ctx, const steel_scene_desc* scenes, uint32_t 
     d.craw = at<float4>(A, s.o_craw); d.con = at<float4>(A, s.o_con); d.ckeys = at<uint4>(A, s.o_ckeys);
     d.rows = at<float4>(A, s.o_rows); d.slots = at<float4>(A, s.o_slots);
     d.pk = at<char>(A, s.o_pk); d.plam = at<float>(A, s.o_plam);
+    d.bpc = at<float4>(A, s.o_bpc);
     d.warm_tab = at<uint32_t>(A, s.o_warm); d.sched = at<uint32_t>(A, s.o_sched);
     d.tw = at<float4>(A, s.o_tw); d.imp = at<float4>(A, s.o_imp); d.aqd = at<float>(A, s.o_aqd);
     d.tscr = at<float>(A, s.o_tscr);

@@ -225,8 +225,8 @@ struct SceneDev {
   float* plam;                       // solve: normal impulses in row order, 0 for rows outside a patch [MAXC]
   uint32_t* warm_tab;                // warm table: 10*WH + 30*AH words
   uint32_t* sched;                   // scheduling arrays, offsets below
-  uint32_t S_UNITOF, S_DSLOT, S_CORDER, S_UKEY, S_USTART0, S_USIZE, S_USTART, S_RK0, S_RK1, S_RK2, S_BPC, S_LEAD,
-      S_KEEP, S_SLOT, S_KEPT, S_ROWOF, S_RUNIT, S_RCON, S_PCOL, S_PORD, S_CSTART, S_META, S_WWIN, S_WSLOT, S_WMASK,
+  uint32_t S_UNITOF, S_DSLOT, S_CORDER, S_UKEY, S_USTART0, S_USIZE, S_USTART, S_RK0, S_RK1, S_RK2, S_LEAD,
+      S_KEEP, S_KEPT, S_ROWOF, S_RUNIT, S_RCON, S_PCOL, S_PORD, S_CSTART, S_META, S_WWIN, S_WSLOT, S_WMASK,
       S_WCOUNT, S_LINKHIT, S_JSPLIT, S_UF, S_UFF, S_UTP, S_DSTART, S_DOFF, S_DLIST, S_BSTART, S_BPOS, S_BREADY,
       S_BLIST, S_RKEY, S_RFLAG, S_WL, S_DFIN, S_DSTATE;
   float4* dhd;                       // solve: dense rows' impulses and scalars in list order [MAXDENSE * 2]
@@ -235,6 +235,7 @@ struct SceneDev {
   // lt[LT_CHL + lt[LT_CHS + l] ...).
   RO<uint32_t> lt;
   uint32_t LT_LVO, LT_LVL, LT_CHS, LT_CHL;
+  float4* bpc;                       // prepare: contact reduction values (plane position, gap, identity) [MAXC]
   float* tscr;                       // per-thread scratch slices (path temporaries), TSCR floats each
   uint32_t TSCR;
   uint32_t TSCR_T;                   // threads the scratch has slices for

@@ -75,25 +75,49 @@ struct Prep {
     return (na < 0 || node_asleep(na)) && (nb < 0 || node_asleep(nb));
   }
 
-  // Twist change of body b for a unit (force, torque) impulse (wgsl.js:1299-1328).
-  __device__ void response(int b, f3 f, f3 t, f3 out[2], bool unsplit = false) const {
-    if (b < 0) { out[0] = sp3(0.0f); out[1] = sp3(0.0f); return; }
-    uint32_t k = bkind(b);
-    if (k == 1u) {
-      float4 q = S.rot[b];
-      m3 R = qmat(q);
-      RO<float4> o = S.sf + S.SF_BODY + (uint32_t)b * 8u;
-      m3 Ii = tr(mcols(v3(o[5]), v3(o[6]), v3(o[7])));
-      out[0] = f * o[0].x;
-      out[1] = mul(R, mul(Ii, mul(tr(R), t)));
+  // Twist change of a body for a unit (force, torque) impulse (wgsl.js:1299-1328). The body's rotation,
+  // inverse inertia and mass are loaded once for all of a row's directions (a row asks each body
+  // six to twelve times); a link answers from its response matrix.
+  struct Body {
+    uint32_t kind;  // 0 static, 1 free, 2 or 3 a link
+    float im;
+    m3 R, Ii;
+    const float* W;
+    const float* W2;  // the unsplit response of kind 2 links; immovable links (kind 3): W
+  };
+  __device__ __forceinline__ Body body(int b) const {
+    Body o;
+    o.kind = 0u;
+    o.im = 0.0f;
+    o.W = o.W2 = nullptr;
+    o.R = o.Ii = mcols(sp3(0.0f), sp3(0.0f), sp3(0.0f));
+    if (b < 0) return o;
+    o.kind = bkind(b);
+    if (o.kind == 1u) {
+      o.R = qmat(S.rot[b]);
+      RO<float4> f = S.sf + S.SF_BODY + (uint32_t)b * 8u;
+      o.Ii = tr(mcols(v3(f[5]), v3(f[6]), v3(f[7])));
+      o.im = f[0].x;
+    } else {
+      const float* L = ar.LB + ar.lo((uint32_t)blink(b));
+      o.W = L + L_W;
+      o.W2 = o.kind == 2u ? L + L_W2 : o.W;
+    }
+    return o;
+  }
+  __device__ __forceinline__ void response(const Body& b, f3 f, f3 t, f3 out[2], bool unsplit = false) const {
+    if (b.kind == 0u) { out[0] = sp3(0.0f); out[1] = sp3(0.0f); return; }
+    if (b.kind == 1u) {
+      out[0] = f * b.im;
+      out[1] = mul(b.R, mul(b.Ii, mul(tr(b.R), t)));
       return;
     }
-    // Kind 2 links answer the unsplit query from L_W2; immovable links (kind 3) from L_W.
-    uint32_t wo = ar.lo((uint32_t)blink(b)) + ((unsplit && k == 2u) ? L_W2 : L_W);
-    const float* W = ar.LB + wo;
+    const float* W = unsplit ? b.W2 : b.W;
     float x[6] = {f.x, f.y, f.z, t.x, t.y, t.z}, o[6];
+#pragma unroll
     for (uint32_t r = 0; r < 6u; r++) {
       float s = 0.0f;
+#pragma unroll
       for (uint32_t c = 0; c < 6u; c++) s += W[r * 6u + c] * x[c];
       o[r] = s;
     }
@@ -164,7 +188,7 @@ struct Prep {
     return i ^ (((i >> 31u) != 0u ? 0xffffffffu : 0u) | 0x80000000u);
   }
   // Slot q's packed (score, identity) (wgsl.js:1498-1503).
-  static __device__ void bp_value(float px, float py, float gap, uint32_t pk, uint32_t q, uint32_t* sc_, uint32_t* id) {
+  static __device__ __forceinline__ void bp_value(float px, float py, float gap, uint32_t pk, uint32_t q, uint32_t* sc_, uint32_t* id) {
     if (q == 6u) { *sc_ = fflip(-gap); *id = pk; return; }
     if (q > 6u && gap > 0.0f) { *sc_ = 0u; *id = 0u; return; }
     const uint32_t k = q > 6u ? q - 7u : q;
@@ -186,6 +210,7 @@ struct Prep {
     float4 qa = make_float4(0, 0, 0, 1);
     if (a >= 0) { ca = v3(S.pos[a]); qa = S.rot[a]; }
     if (b >= 0) cb = v3(S.pos[b]);
+    const Body Ba = body(a), Bb = body(b);
     float r = fmx(fmn(bradius(a), bradius(b)), 1e-4f);
     uint32_t seed = st;
     for (uint32_t i = st; i < st + n; i++) if (rows[i * ROWS + 1u].w < rows[seed * ROWS + 1u].w) seed = i;
@@ -282,8 +307,8 @@ struct Prep {
       f3 Ma[2][2], Mb[2][2];
       f3 dirs[2] = {t1, t2};
       for (uint32_t q = 0; q < 2u; q++) {
-        response(a, -dirs[q], -cross(fra, dirs[q]), Ma[q]);
-        response(b, dirs[q], cross(frb, dirs[q]), Mb[q]);
+        response(Ba, -dirs[q], -cross(fra, dirs[q]), Ma[q]);
+        response(Bb, dirs[q], cross(frb, dirs[q]), Mb[q]);
         rows[o + 11u + q * 4u] = mf4(Ma[q][0], 0.0f);
         rows[o + 12u + q * 4u] = mf4(Ma[q][1], 0.0f);
         rows[o + 13u + q * 4u] = mf4(Mb[q][0], 0.0f);
@@ -378,8 +403,8 @@ struct Prep {
     const float mu = rows[seed * ROWS + 2u].w;
     if (r <= 0.0f || mu <= 0.0f) { rows[L + TO] = make_float4(0, 0, 0, 0); return; }
     f3 Ma[2], Mb[2];
-    response(a, sp3(0.0f), -ns, Ma);
-    response(b, sp3(0.0f), ns, Mb);
+    response(body(a), sp3(0.0f), -ns, Ma);
+    response(body(b), sp3(0.0f), ns, Mb);
     const float k = dot(-ns, Ma[1]) + dot(ns, Mb[1]);
     const float lead = rows[L + TO + 4u].w;
     rows[L + TO] = mf4(Ma[0], mu);
@@ -423,18 +448,22 @@ struct Prep {
     uint32_t o = idx * ROWS;
     f3 dirs[3] = {n, t1, t2};
     f3 Ma[3][2], Mb[3][2];
+    const Body Ba = body(a), Bb = body(b);
+#pragma unroll
     for (uint32_t r = 0; r < 3u; r++) {
       f3 d = dirs[r];
       f3 aa = r == 0u ? ra : fa, ab = r == 0u ? rb : fb;
-      response(a, -d, -cross(aa, d), Ma[r]);
-      response(b, d, cross(ab, d), Mb[r]);
+      response(Ba, -d, -cross(aa, d), Ma[r]);
+      response(Bb, d, cross(ab, d), Mb[r]);
       rows[o + 7u + r * 4u] = mf4(Ma[r][0], 0.0f);
       rows[o + 8u + r * 4u] = mf4(Ma[r][1], 0.0f);
       rows[o + 9u + r * 4u] = mf4(Mb[r][0], 0.0f);
       rows[o + 10u + r * 4u] = mf4(Mb[r][1], 0.0f);
     }
     float K[9];
+#pragma unroll
     for (uint32_t r = 0; r < 3u; r++)
+#pragma unroll
       for (uint32_t s = 0; s < 3u; s++) {
         f3 d = dirs[r];
         f3 aa = r == 0u ? ra : fa, ab = r == 0u ? rb : fb;
@@ -501,8 +530,8 @@ struct Prep {
     float wrow = row_weight(phi);
     if (wrow < 1.0f && ((a >= 0 && bkind(a) == 2u) || (b >= 0 && bkind(b) == 2u))) {
       f3 ua[2], ub[2];
-      response(a, -n, -cross(ra, n), ua, true);
-      response(b, n, cross(rb, n), ub, true);
+      response(Ba, -n, -cross(ra, n), ua, true);
+      response(Bb, n, cross(rb, n), ub, true);
       float du = ((dot(-n, ua[0]) + dot(-cross(ra, n), ua[1])) + dot(n, ub[0])) + dot(cross(rb, n), ub[1]);
       if (du > 0.0f && K[0] != du) wrow = (wrow * K[0]) / (wrow * K[0] + (1.0f - wrow) * du);
     }
@@ -515,8 +544,8 @@ struct Prep {
       f3 MA[3][2], MB[3][2];
       for (uint32_t r = 0; r < 3u; r++) {
         const f3 d = dirs[r];
-        response(a, sp3(0.0f), -d, MA[r]);
-        response(b, sp3(0.0f), d, MB[r]);
+        response(Ba, sp3(0.0f), -d, MA[r]);
+        response(Bb, sp3(0.0f), d, MB[r]);
         rows[o + 22u + r * 4u] = mf4(MA[r][0], 0.0f);
         rows[o + 23u + r * 4u] = mf4(MA[r][1], 0.0f);
         rows[o + 24u + r * 4u] = mf4(MB[r][0], 0.0f);
@@ -922,9 +951,6 @@ __device__ __forceinline__ void prepare_scene(const BatchDev& B, uint32_t sc, Te
   uint32_t nu = 0u, nl = 0u, ndc = 0u;
   if (b0) {
     const uint32_t tid = threadIdx.x, nt = blockDim.x;
-    const uint32_t ch = (nc + nt - 1u) / nt;
-    const uint32_t c_lo = min(tid * ch, nc), c_hi = min(c_lo + ch, nc);
-    uint32_t heads = 0u, listed = 0u, dn = 0u;
     auto pair_of = [&](uint32_t c) {
       float4 m = S.con[c * 5u + 2u];
       return (uint32_t)(f2i(m.x) + 1) | ((uint32_t)(f2i(m.y) + 1) << 16u);
@@ -941,43 +967,43 @@ __device__ __forceinline__ void prepare_scene(const BatchDev& B, uint32_t sc, Te
       float4 m = S.con[c * 5u + 2u];
       return pr.pair_asleep(f2i(m.x), f2i(m.y));
     };
-    for (uint32_t c = c_lo; c < c_hi; c++) {
-      if (asleep(c)) continue;
-      if (is_dense(c)) { dn++; continue; }
-      listed++;
-      if (c == 0u || pair_of(c - 1u) != pair_of(c)) heads++;
-    }
-    uint32_t ubase = block_excl_scan(heads, stmp, &nu);
-    uint32_t lbase = block_excl_scan(listed, stmp, &nl);
-    uint32_t dbase = block_excl_scan(dn, stmp, &ndc);
-    {
-      uint32_t unit = ubase, pos = lbase, ds = dbase;
-      for (uint32_t c = c_lo; c < c_hi; c++) {
-        if (asleep(c)) {
-          sch[S.S_UNITOF + c] = 0xffffffffu;
-          sch[S.S_DSLOT + c] = 0xffffffffu;
-          continue;
+    // A contact per thread and tile, in order: one scan of the three counts (units, listed contacts,
+    // dense contacts, 10 bits each: a tile has at most 512) places the tile's. With a run of contacts
+    // per thread each thread's loads were a serial chain (24 contacts a thread on a 700-body pile:
+    // 220,000 cycles).
+    for (uint32_t c0 = 0; c0 < nc; c0 += nt) {
+      const uint32_t c = c0 + tid;
+      uint32_t pk = 0u;
+      bool head = false, list = false, dense = false;
+      if (c < nc && !asleep(c)) {
+        dense = is_dense(c);
+        if (!dense) {
+          list = true;
+          pk = pair_of(c);
+          head = c == 0u || pair_of(c - 1u) != pk;
         }
-        if (is_dense(c)) {
-          sch[S.S_UNITOF + c] = 0xffffffffu;
-          sch[S.S_DSLOT + c] = ds++;
-          continue;
-        }
-        sch[S.S_DSLOT + c] = 0xffffffffu;
-        uint32_t pk = pair_of(c);
-        if (c == 0u || pair_of(c - 1u) != pk) {
-          sch[S.S_UKEY + unit] = pk;
-          sch[S.S_USTART0 + unit] = pos;
-          unit++;
-        }
-        sch[S.S_UNITOF + c] = unit - 1u;
-        sch[S.S_CORDER + pos] = c;
-        pos++;
-        float4 m = S.con[c * 5u + 2u];
-        int a = f2i(m.x), b = f2i(m.y);
-        if (a >= 0 && pr.bkind(a) == 2u) sch[S.S_LINKHIT + a] = 1u;
-        if (b >= 0 && pr.bkind(b) == 2u) sch[S.S_LINKHIT + b] = 1u;
       }
+      uint32_t total;
+      const uint32_t at = block_excl_scan((head ? 1u : 0u) | (list ? 1u << 10u : 0u) | (dense ? 1u << 20u : 0u), stmp, &total);
+      if (c < nc) {
+        // The contact's unit is the last head at or before it.
+        const uint32_t unit = nu + (at & 1023u) + (head ? 1u : 0u) - 1u, pos = nl + ((at >> 10u) & 1023u);
+        sch[S.S_DSLOT + c] = dense ? ndc + (at >> 20u) : 0xffffffffu;
+        sch[S.S_UNITOF + c] = list ? unit : 0xffffffffu;
+        if (list) {
+          if (head) {
+            sch[S.S_UKEY + unit] = pk;
+            sch[S.S_USTART0 + unit] = pos;
+          }
+          sch[S.S_CORDER + pos] = c;
+          const int a = (int)(pk & 0xffffu) - 1, b = (int)(pk >> 16u) - 1;
+          if (a >= 0 && pr.bkind(a) == 2u) sch[S.S_LINKHIT + a] = 1u;
+          if (b >= 0 && pr.bkind(b) == 2u) sch[S.S_LINKHIT + b] = 1u;
+        }
+      }
+      nu += total & 1023u;
+      nl += (total >> 10u) & 1023u;
+      ndc += total >> 20u;
     }
     if (tid == 0u) sch[S.S_USTART0 + nu] = nl;
     if (TEAM && tid == 0u) { B.team_bar[4] = nu; B.team_bar[5] = nl; B.team_bar[6] = ndc; }
@@ -1012,56 +1038,69 @@ __device__ __forceinline__ void prepare_scene(const BatchDev& B, uint32_t sc, Te
       }
     }
   }
-  // Phase 5: body-pair contact reduction over each unit's listed contacts.
+  // Phase 5: body-pair contact reduction over each unit's listed contacts. A contact group keeps the
+  // contacts that are extreme in one of 13 slots. A group is found by its first contact's thread,
+  // which takes the slots' maxima over its contacts and marks the winners; a contact alone in its
+  // unit or group wins every slot. (Most are: going through slot words in memory, 26 atomic maxima a
+  // contact, this took 540 us of a 700-body pile's prepare.)
   for (uint32_t p = tid; p < nl; p += nt) {
+    const uint32_t u = sch[S.S_UNITOF + sch[S.S_CORDER + p]];
+    if (S.COMPL == 1u || sch[S.S_USIZE + u] < 2u) {  // compliant contacts stay whole
+      sch[S.S_KEEP + p] = 1u;
+      sch[S.S_LEAD + p] = 0xffffffffu;
+      continue;
+    }
     uint32_t k[3], pk;
     float px, py, gap;
     pr.bp_contact(sch[S.S_CORDER + p], k, &px, &py, &gap, &pk);
     sch[S.S_RK0 + p] = k[0]; sch[S.S_RK1 + p] = k[1]; sch[S.S_RK2 + p] = k[2];
-    uint32_t* bpc = sch + S.S_BPC + p * 4u;
-    bpc[0] = __float_as_uint(px); bpc[1] = __float_as_uint(py); bpc[2] = __float_as_uint(gap); bpc[3] = pk;
+    sch[S.S_LEAD + p] = u;
+    S.bpc[p] = make_float4(px, py, gap, __uint_as_float(pk));
   }
   tm.sync();
   for (uint32_t p = tid; p < nl; p += nt) {
-    uint32_t st = sch[S.S_USTART0 + sch[S.S_UNITOF + sch[S.S_CORDER + p]]];
-    uint32_t k0 = sch[S.S_RK0 + p], k1 = sch[S.S_RK1 + p], k2 = sch[S.S_RK2 + p];
-    uint32_t lead = p;
-    for (uint32_t m = st; m < p; m++)
-      if (sch[S.S_RK2 + m] == k2 && sch[S.S_RK0 + m] == k0 && sch[S.S_RK1 + m] == k1) { lead = m; break; }
-    sch[S.S_LEAD + p] = lead;
-    for (uint32_t q = 0; q < 26u; q++) sch[S.S_SLOT + p * 26u + q] = 0u;
-  }
-  tm.sync();
-  for (uint32_t p = tid; p < nl; p += nt) {
-    const uint32_t* bpc = sch + S.S_BPC + p * 4u;
-    uint32_t* sl = sch + S.S_SLOT + sch[S.S_LEAD + p] * 26u;
-    for (uint32_t q = 0; q < 13u; q++) {
-      uint32_t s_, id;
-      Prep::bp_value(__uint_as_float(bpc[0]), __uint_as_float(bpc[1]), __uint_as_float(bpc[2]), bpc[3], q, &s_, &id);
-      if (id != 0u) atomicMax(&sl[q * 2u], s_);
+    const uint32_t u = sch[S.S_LEAD + p];
+    if (u == 0xffffffffu) continue;
+    const uint32_t st = sch[S.S_USTART0 + u], en = st + sch[S.S_USIZE + u];
+    const uint32_t k0 = sch[S.S_RK0 + p], k1 = sch[S.S_RK1 + p], k2 = sch[S.S_RK2 + p];
+    auto same = [&](uint32_t m) { return sch[S.S_RK2 + m] == k2 && sch[S.S_RK0 + m] == k0 && sch[S.S_RK1 + m] == k1; };
+    bool first = true;
+    for (uint32_t m = st; m < p && first; m++) first = !same(m);
+    if (!first) continue;
+    uint32_t members = 1u;
+    for (uint32_t m = p + 1u; m < en; m++) members += same(m) ? 1u : 0u;
+    if (members == 1u) {
+      sch[S.S_KEEP + p] = 1u;
+      continue;
     }
-  }
-  tm.sync();
-  for (uint32_t p = tid; p < nl; p += nt) {
-    const uint32_t* bpc = sch + S.S_BPC + p * 4u;
-    uint32_t* sl = sch + S.S_SLOT + sch[S.S_LEAD + p] * 26u;
-    for (uint32_t q = 0; q < 13u; q++) {
-      uint32_t s_, id;
-      Prep::bp_value(__uint_as_float(bpc[0]), __uint_as_float(bpc[1]), __uint_as_float(bpc[2]), bpc[3], q, &s_, &id);
-      if (id != 0u && s_ == sl[q * 2u]) atomicMax(&sl[q * 2u + 1u], id);
+    uint32_t bs[13], bi[13];
+#pragma unroll
+    for (uint32_t q = 0; q < 13u; q++) { bs[q] = 0u; bi[q] = 0u; }
+    for (uint32_t m = p; m < en; m++) {
+      if (m != p && !same(m)) continue;
+      const float4 v = S.bpc[m];
+#pragma unroll
+      for (uint32_t q = 0; q < 13u; q++) {
+        uint32_t s_, id;
+        Prep::bp_value(v.x, v.y, v.z, __float_as_uint(v.w), q, &s_, &id);
+        if (id != 0u && s_ >= bs[q]) {
+          bi[q] = s_ > bs[q] ? id : max(bi[q], id);
+          bs[q] = s_;
+        }
+      }
     }
-  }
-  tm.sync();
-  for (uint32_t p = tid; p < nl; p += nt) {
-    const uint32_t* bpc = sch + S.S_BPC + p * 4u;
-    const uint32_t* sl = sch + S.S_SLOT + sch[S.S_LEAD + p] * 26u;
-    bool win = false;
-    for (uint32_t q = 0; q < 13u; q++) {
-      uint32_t s_, id;
-      Prep::bp_value(__uint_as_float(bpc[0]), __uint_as_float(bpc[1]), __uint_as_float(bpc[2]), bpc[3], q, &s_, &id);
-      if (id != 0u && s_ == sl[q * 2u] && id == sl[q * 2u + 1u]) win = true;
+    for (uint32_t m = p; m < en; m++) {
+      if (m != p && !same(m)) continue;
+      const float4 v = S.bpc[m];
+      bool win = false;
+#pragma unroll
+      for (uint32_t q = 0; q < 13u; q++) {
+        uint32_t s_, id;
+        Prep::bp_value(v.x, v.y, v.z, __float_as_uint(v.w), q, &s_, &id);
+        win = win || (id != 0u && s_ == bs[q] && id == bi[q]);
+      }
+      sch[S.S_KEEP + m] = win ? 1u : 0u;
     }
-    sch[S.S_KEEP + p] = (win || S.COMPL == 1u) ? 1u : 0u;  // compliant contacts stay whole
   }
   tm.sync();
   for (uint32_t u = tid; u < nu; u += nt) {
