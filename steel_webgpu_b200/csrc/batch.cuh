@@ -76,7 +76,7 @@ constexpr uint32_t blocks_per_sm_of(uint32_t threads) { return 65536u / (threads
 
 // Device error codes written to BatchDev::error.
 enum : uint32_t { ERR_NONE = 0, ERR_SORT_CAPACITY = 1, ERR_JOB_CAPACITY = 2, ERR_STAGE_TIMEOUT = 3, ERR_SORT_TIMEOUT = 4,
-                  ERR_TEAM_TIMEOUT = 5 };
+                  ERR_TEAM_TIMEOUT = 5, ERR_COLOR_TIMEOUT = 6 };
 
 // Contact sort of scenes whose padded keys may exceed the block sort's shared array
 // (next_pow2(MAXC) > SORT_SMEM_KEYS): a device-wide LSD radix sort, onesweep style (one histogram
@@ -91,6 +91,7 @@ constexpr uint32_t RS_TILE = RS_THREADS * RS_ITEMS;
 constexpr uint32_t RS_DIGITS = 12;          // 96 key bits, 8 per digit
 constexpr uint32_t RS_SPIN_LIMIT = 1u << 22;  // polls of a preceding tile's status before giving up
 constexpr uint32_t TEAM_WAIT_LIMIT = 1u << 22;  // polls of a team launch's grid barrier before giving up
+constexpr uint32_t COLOR_WAIT_LIMIT = 1u << 22;  // passes of a thread over its bodies' frontiers before giving up
 // Team launches (team.cuh) on a batch of one scene: the default takes scenes of at least
 // TEAM_MIN_BODIES bodies or TEAM_MIN_ARTS articulations; such a scene's per-thread scratch has
 // slices for TEAM_SCRATCH_BLOCKS blocks, so the prepare's scratch passes spread over that many.
@@ -118,6 +119,10 @@ constexpr uint32_t STAGE_WMASK_CAP = 16u * 1024u;  // per-body color masks (NB *
 constexpr size_t SMEM_PER_SM = 228u * 1024u;
 constexpr size_t solve_smem_room(uint32_t resident) {
   return (SMEM_PER_SM / (resident > 0u ? resident : 1u) - 6u * 1024u) & ~(size_t)127u;
+}
+// The same for prepare blocks, whose static arrays are larger (under 11 KB).
+constexpr size_t prep_smem_room(uint32_t resident) {
+  return (SMEM_PER_SM / (resident > 0u ? resident : 1u) - 12u * 1024u) & ~(size_t)127u;
 }
 // Percent of an SM's shared memory that a solve launch's resident blocks use.
 inline unsigned int solve_carveout(const BatchDev& b) {

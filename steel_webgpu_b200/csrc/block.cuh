@@ -4,6 +4,20 @@
 
 namespace steel {
 
+// Loads and stores between the threads of a block without barriers (generic addresses).
+SD uint32_t ld_acquire_cta(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.acquire.cta.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+SD uint32_t ld_relaxed_cta(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.cta.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+SD void st_relaxed_cta(uint32_t* p, uint32_t v) { asm volatile("st.relaxed.cta.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
+SD void st_release_cta(uint32_t* p, uint32_t v) { asm volatile("st.release.cta.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
+
 // Exclusive prefix sum of v over the block's threads, in thread order; *total gets the sum.
 // tmp: shared memory of at least 33 words. All threads must call it.
 SD uint32_t block_excl_scan(uint32_t v, uint32_t* tmp, uint32_t* total) {

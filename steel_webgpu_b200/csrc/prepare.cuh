@@ -1160,106 +1160,203 @@ __device__ __forceinline__ void prepare_scene(const BatchDev& B, uint32_t sc, Te
       if (stage & STAGE_WMASK)
         for (uint32_t i = tid; i < S.NB * NCOLW; i += nt) wmask[i] = 0u;
       if (S.LONGEST_FIRST == 0u) {
-        // First-fit in row order, in parallel rounds with the same colors (Jones-Plassmann with the
-        // row index as priority). Every body keeps its rows in row order and a frontier, the first
+        // First-fit in row order, with the same colors from many threads (Jones-Plassmann with the row
+        // index as priority). Every body lists its rows in row order and keeps a frontier, the first
         // of them not yet colored; rows on one body are colored in that order, so when a row is the
         // frontier of both its bodies every earlier row touching them has its color, and the body
-        // masks hold exactly the colors the serial pass would see. Such rows share no body, so one
-        // round colors all of them without conflicts. A round only looks at the bodies whose
-        // frontier moved in the previous one (all bodies in the first): phase A finds the ready rows
-        // among their frontier rows (a row whose two bodies both look at it is listed once), phase B
-        // colors them, advances the frontiers and lists the moved bodies for the next round. A row
-        // is found in the round its last frontier reaches it, since that body is on the list. Each
-        // round colors at least the lowest uncolored row, so the rounds end.
-        uint32_t* bstart = sch + S.S_BSTART;  // [NB + 1] each body's first list entry
-        uint32_t* bpos = sch + S.S_BPOS;      // [NB] fill cursor, then frontier
-        uint32_t* rdy = sch + S.S_BREADY;     // [NB] rows found ready in a round
-        uint32_t* blist = sch + S.S_BLIST;    // [2 * MAXC] rows of each body
-        uint32_t* rkey = sch + S.S_RKEY;      // [MAXC] body-pair key of each row
-        uint32_t* rflag = sch + S.S_RFLAG;    // [MAXC] the row is on the ready list
-        uint32_t* wl[2] = {sch + S.S_WL, sch + S.S_WL + S.NB};  // [2][NB] bodies to look at
-        __shared__ uint32_t wl_n[2], rdy_n;
+        // masks hold exactly the colors the serial pass would see. A row is colored by the thread of
+        // its lower body, which then moves both frontiers on. The threads go over their bodies without
+        // barriers: a body's masks are written before its frontier moves (release) and read after
+        // it is seen to have (acquire), and the lowest uncolored row is always ready, so every pass of
+        // its thread colors it. On 64 boxes this took the prepare from 166 to 140 us. It needs the
+        // lists in shared memory, beyond the scene's staging (from global memory the acquiring loads
+        // made an 8192-body pile's prepare 2.44 ms against 1.64 ms); other scenes take the rounds
+        // below.
         const uint32_t NB = S.NB;
-        for (uint32_t b = tid; b <= NB; b += nt) bstart[b] = 0u;
-        if (tid == 0u) { wl_n[0] = 0u; wl_n[1] = 0u; rdy_n = 0u; }
-        __syncthreads();
-        for (uint32_t r = tid; r < total; r += nt) {
-          const uint32_t key = sch[S.S_UKEY + sch[S.S_RUNIT + r]];
-          rkey[r] = key;
-          rflag[r] = 0u;
-          const int a = (int)(key & 0xffffu) - 1, b = (int)(key >> 16u) - 1;
-          if (a >= 0) atomicAdd(&bstart[a], 1u);
-          if (b >= 0 && b != a) atomicAdd(&bstart[b], 1u);
-        }
-        __syncthreads();
-        block_scan_array(bstart, NB + 1u, stmp);
-        for (uint32_t b = tid; b < NB; b += nt) bpos[b] = bstart[b];
-        __syncthreads();
-        for (uint32_t r = tid; r < total; r += nt) {
-          const uint32_t key = rkey[r];
-          const int a = (int)(key & 0xffffu) - 1, b = (int)(key >> 16u) - 1;
-          if (a >= 0) blist[atomicAdd(&bpos[a], 1u)] = r;
-          if (b >= 0 && b != a) blist[atomicAdd(&bpos[b], 1u)] = r;
-        }
-        __syncthreads();
-        for (uint32_t b = tid; b < NB; b += nt) {  // each body's rows in row order
-          const uint32_t s0 = bstart[b], s1 = bstart[b + 1u];
-          for (uint32_t i = s0 + 1u; i < s1; i++) {
-            const uint32_t v = blist[i];
-            uint32_t j = i;
-            while (j > s0 && blist[j - 1u] > v) { blist[j] = blist[j - 1u]; j--; }
-            blist[j] = v;
-          }
-          bpos[b] = s0;
-          if (s1 > s0) wl[0][atomicAdd(&wl_n[0], 1u)] = b;
-        }
-        __syncthreads();
-        uint32_t cur = 0u;
-        for (uint32_t round = 0; round <= total; round++) {
-          const uint32_t n = wl_n[cur];
-          if (n == 0u) break;  // the same value in every thread (read after the last barrier)
-          for (uint32_t i = tid; i < n; i += nt) {
-            const uint32_t b = wl[cur][i];
-            const uint32_t p = bpos[b];
-            if (p >= bstart[b + 1u]) continue;
-            const uint32_t r = blist[p];
-            const uint32_t key = rkey[r];
-            const int x = (int)(key & 0xffffu) - 1, y = (int)(key >> 16u) - 1;
-            const int other = x == (int)b ? y : x;
-            if (other >= 0 && other != (int)b && blist[bpos[other]] != r) continue;
-            if (atomicExch(&rflag[r], 1u) == 0u) rdy[atomicAdd(&rdy_n, 1u)] = r;
+        const uint32_t lists_at = (lay.total + 15u) & ~15u;
+        if (total < 65536u && lists_at + 4ull * (2ull * NB + 2ull) + 8ull * total + 8ull <= B.prep_smem) {
+          uint32_t* bstart = reinterpret_cast<uint32_t*>(pb + lists_at);             // [NB + 1] first list entry
+          uint32_t* bpos = bstart + NB + 1u;                                         // [NB] fill cursor, frontier
+          uint16_t* blist = reinterpret_cast<uint16_t*>(bpos + NB + 1u);             // [2 * rows] rows of each body
+          uint16_t* bother = blist + 2u * total;                                     // the row's other body, or -1
+          for (uint32_t b = tid; b <= NB; b += nt) bstart[b] = 0u;
+          __syncthreads();
+          auto pair_of_row = [&](uint32_t r, int& a, int& b) {
+            const uint32_t key = sch[S.S_UKEY + sch[S.S_RUNIT + r]];
+            a = (int)(key & 0xffffu) - 1;
+            b = (int)(key >> 16u) - 1;
+          };
+          for (uint32_t r = tid; r < total; r += nt) {
+            int a, b;
+            pair_of_row(r, a, b);
+            sch[S.S_PCOL + r] = S.NCOL;
+            if (a >= 0) atomicAdd(&bstart[a], 1u);
+            if (b >= 0 && b != a) atomicAdd(&bstart[b], 1u);
           }
           __syncthreads();
-          const uint32_t nr = rdy_n;
-          if (tid == 0u) wl_n[cur ^ 1u] = 0u;
+          block_scan_array(bstart, NB + 1u, stmp);
+          for (uint32_t b = tid; b < NB; b += nt) bpos[b] = bstart[b];
           __syncthreads();
-          for (uint32_t k = tid; k < nr; k += nt) {
-            const uint32_t r = rdy[k];
-            const uint32_t key = rkey[r];
-            const int a = (int)(key & 0xffffu) - 1, c = (int)(key >> 16u) - 1;
-            uint32_t col = S.NCOL;
-            for (uint32_t w = 0; w < NCOLW; w++) {
-              uint32_t used = 0u;
-              if (a >= 0) used |= wmask[(uint32_t)a * NCOLW + w];
-              if (c >= 0) used |= wmask[(uint32_t)c * NCOLW + w];
-              if (used != 0xffffffffu) {
-                uint32_t kk = (uint32_t)__ffs(~used) - 1u;
-                if (a >= 0) wmask[(uint32_t)a * NCOLW + w] |= 1u << kk;
-                if (c >= 0) wmask[(uint32_t)c * NCOLW + w] |= 1u << kk;
-                col = w * 32u + kk;
-                break;
+          for (uint32_t r = tid; r < total; r += nt) {
+            int a, b;
+            pair_of_row(r, a, b);
+            if (a >= 0) blist[atomicAdd(&bpos[a], 1u)] = (uint16_t)r;
+            if (b >= 0 && b != a) blist[atomicAdd(&bpos[b], 1u)] = (uint16_t)r;
+          }
+          __syncthreads();
+          for (uint32_t b = tid; b < NB; b += nt) {  // each body's rows in row order
+            const uint32_t s0 = bstart[b], s1 = bstart[b + 1u];
+            for (uint32_t i = s0 + 1u; i < s1; i++) {
+              const uint16_t v = blist[i];
+              uint32_t j = i;
+              while (j > s0 && blist[j - 1u] > v) { blist[j] = blist[j - 1u]; j--; }
+              blist[j] = v;
+            }
+            for (uint32_t i = s0; i < s1; i++) {
+              int x, y;
+              pair_of_row(blist[i], x, y);
+              const int o = x == (int)b ? y : x;
+              bother[i] = o == (int)b ? (uint16_t)0xffffu : (uint16_t)o;
+            }
+            bpos[b] = s0;
+          }
+          __syncthreads();
+          uint32_t passes = 0u;
+          for (bool left = true; left;) {
+            left = false;
+            for (uint32_t b = tid; b < NB; b += nt) {
+              const uint32_t end = bstart[b + 1u];
+              // A few rows of the body in a row while they are ready (its contacts with static bodies are).
+              for (uint32_t k = 0; k < 4u; k++) {
+                const uint32_t p = ld_acquire_cta(&bpos[b]);
+                if (p >= end) break;
+                left = true;
+                const uint32_t r = blist[p], o = bother[p];
+                uint32_t po = 0u;
+                if (o != 0xffffu) {
+                  if (o < b) break;  // the lower body's thread colors it
+                  po = ld_acquire_cta(&bpos[o]);
+                  if (blist[po] != r) break;
+                }
+                uint32_t col = S.NCOL;
+                for (uint32_t w = 0; w < NCOLW; w++) {
+                  uint32_t used = ld_relaxed_cta(&wmask[b * NCOLW + w]);
+                  const uint32_t other = o != 0xffffu ? ld_relaxed_cta(&wmask[o * NCOLW + w]) : 0u;
+                  if ((used | other) != 0xffffffffu) {
+                    const uint32_t bit = ~(used | other) & (0u - ~(used | other));
+                    st_relaxed_cta(&wmask[b * NCOLW + w], used | bit);
+                    if (o != 0xffffu) st_relaxed_cta(&wmask[o * NCOLW + w], other | bit);
+                    col = w * 32u + (uint32_t)__ffs(bit) - 1u;
+                    break;
+                  }
+                }
+                sch[S.S_PCOL + r] = col;
+                st_release_cta(&bpos[b], p + 1u);
+                if (o != 0xffffu) st_release_cta(&bpos[o], po + 1u);
               }
             }
-            sch[S.S_PCOL + r] = col;
-            atomicAdd(&wcount[col], 1u);
-            // Advance the frontiers; a body with rows left is looked at in the next round.
-            if (a >= 0 && ++bpos[a] < bstart[a + 1u]) wl[cur ^ 1u][atomicAdd(&wl_n[cur ^ 1u], 1u)] = (uint32_t)a;
-            if (c >= 0 && c != a && ++bpos[c] < bstart[c + 1u]) wl[cur ^ 1u][atomicAdd(&wl_n[cur ^ 1u], 1u)] = (uint32_t)c;
+            if (left && ++passes >= COLOR_WAIT_LIMIT) {
+              atomicCAS(B.error, 0u, (uint32_t)ERR_COLOR_TIMEOUT);
+              break;  // the rows left keep the overflow color
+            }
           }
           __syncthreads();
-          if (tid == 0u) rdy_n = 0u;
-          cur ^= 1u;
+          for (uint32_t r = tid; r < total; r += nt) atomicAdd(&wcount[sch[S.S_PCOL + r]], 1u);
+        } else {
+          // Parallel rounds: a round only looks at the bodies whose frontier moved in the previous one
+          // (all bodies in the first): phase A finds the ready rows among their frontier rows (a row
+          // whose two bodies both look at it is listed once), phase B colors them, advances the
+          // frontiers and lists the moved bodies for the next round. Each round colors at least the
+          // lowest uncolored row, so the rounds end.
+          uint32_t* bstart = sch + S.S_BSTART;  // [NB + 1] each body's first list entry
+          uint32_t* bpos = sch + S.S_BPOS;      // [NB] fill cursor, then frontier
+          uint32_t* rdy = sch + S.S_BREADY;     // [NB] rows found ready in a round
+          uint32_t* blist = sch + S.S_BLIST;    // [2 * MAXC] rows of each body
+          uint32_t* rkey = sch + S.S_RKEY;      // [MAXC] body-pair key of each row
+          uint32_t* rflag = sch + S.S_RFLAG;    // [MAXC] the row is on the ready list
+          uint32_t* wl[2] = {sch + S.S_WL, sch + S.S_WL + S.NB};  // [2][NB] bodies to look at
+          __shared__ uint32_t wl_n[2], rdy_n;
+          for (uint32_t b = tid; b <= NB; b += nt) bstart[b] = 0u;
+          if (tid == 0u) { wl_n[0] = 0u; wl_n[1] = 0u; rdy_n = 0u; }
           __syncthreads();
+          for (uint32_t r = tid; r < total; r += nt) {
+            const uint32_t key = sch[S.S_UKEY + sch[S.S_RUNIT + r]];
+            rkey[r] = key;
+            rflag[r] = 0u;
+            const int a = (int)(key & 0xffffu) - 1, b = (int)(key >> 16u) - 1;
+            if (a >= 0) atomicAdd(&bstart[a], 1u);
+            if (b >= 0 && b != a) atomicAdd(&bstart[b], 1u);
+          }
+          __syncthreads();
+          block_scan_array(bstart, NB + 1u, stmp);
+          for (uint32_t b = tid; b < NB; b += nt) bpos[b] = bstart[b];
+          __syncthreads();
+          for (uint32_t r = tid; r < total; r += nt) {
+            const uint32_t key = rkey[r];
+            const int a = (int)(key & 0xffffu) - 1, b = (int)(key >> 16u) - 1;
+            if (a >= 0) blist[atomicAdd(&bpos[a], 1u)] = r;
+            if (b >= 0 && b != a) blist[atomicAdd(&bpos[b], 1u)] = r;
+          }
+          __syncthreads();
+          for (uint32_t b = tid; b < NB; b += nt) {  // each body's rows in row order
+            const uint32_t s0 = bstart[b], s1 = bstart[b + 1u];
+            for (uint32_t i = s0 + 1u; i < s1; i++) {
+              const uint32_t v = blist[i];
+              uint32_t j = i;
+              while (j > s0 && blist[j - 1u] > v) { blist[j] = blist[j - 1u]; j--; }
+              blist[j] = v;
+            }
+            bpos[b] = s0;
+            if (s1 > s0) wl[0][atomicAdd(&wl_n[0], 1u)] = b;
+          }
+          __syncthreads();
+          uint32_t cur = 0u;
+          for (uint32_t round = 0; round <= total; round++) {
+            const uint32_t n = wl_n[cur];
+            if (n == 0u) break;  // the same value in every thread (read after the last barrier)
+            for (uint32_t i = tid; i < n; i += nt) {
+              const uint32_t b = wl[cur][i];
+              const uint32_t p = bpos[b];
+              if (p >= bstart[b + 1u]) continue;
+              const uint32_t r = blist[p];
+              const uint32_t key = rkey[r];
+              const int x = (int)(key & 0xffffu) - 1, y = (int)(key >> 16u) - 1;
+              const int other = x == (int)b ? y : x;
+              if (other >= 0 && other != (int)b && blist[bpos[other]] != r) continue;
+              if (atomicExch(&rflag[r], 1u) == 0u) rdy[atomicAdd(&rdy_n, 1u)] = r;
+            }
+            __syncthreads();
+            const uint32_t nr = rdy_n;
+            if (tid == 0u) wl_n[cur ^ 1u] = 0u;
+            __syncthreads();
+            for (uint32_t k = tid; k < nr; k += nt) {
+              const uint32_t r = rdy[k];
+              const uint32_t key = rkey[r];
+              const int a = (int)(key & 0xffffu) - 1, c = (int)(key >> 16u) - 1;
+              uint32_t col = S.NCOL;
+              for (uint32_t w = 0; w < NCOLW; w++) {
+                uint32_t used = 0u;
+                if (a >= 0) used |= wmask[(uint32_t)a * NCOLW + w];
+                if (c >= 0) used |= wmask[(uint32_t)c * NCOLW + w];
+                if (used != 0xffffffffu) {
+                  uint32_t kk = (uint32_t)__ffs(~used) - 1u;
+                  if (a >= 0) wmask[(uint32_t)a * NCOLW + w] |= 1u << kk;
+                  if (c >= 0) wmask[(uint32_t)c * NCOLW + w] |= 1u << kk;
+                  col = w * 32u + kk;
+                  break;
+                }
+              }
+              sch[S.S_PCOL + r] = col;
+              atomicAdd(&wcount[col], 1u);
+              // Advance the frontiers; a body with rows left is looked at in the next round.
+              if (a >= 0 && ++bpos[a] < bstart[a + 1u]) wl[cur ^ 1u][atomicAdd(&wl_n[cur ^ 1u], 1u)] = (uint32_t)a;
+              if (c >= 0 && c != a && ++bpos[c] < bstart[c + 1u]) wl[cur ^ 1u][atomicAdd(&wl_n[cur ^ 1u], 1u)] = (uint32_t)c;
+            }
+            __syncthreads();
+            if (tid == 0u) rdy_n = 0u;
+            cur ^= 1u;
+            __syncthreads();
+          }
         }
       }
       __syncthreads();
