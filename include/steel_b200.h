@@ -119,8 +119,9 @@ int steel_set_graph(steel_batch* b, int enabled);
    groups of about equal size whose launch sequences run on parallel streams (branches of the frame
    graph), so one group's kernels use the SMs another group's kernel tails leave idle (0 or 1: one
    sequence; the serving loop always uses one). A batch starts at 512 threads when it has no more
-   scenes than SMs (the per-thread scratch is sized for that), else at 128, which is also the
-   largest block it accepts. Results are the same bits under every configuration. */
+   scenes than SMs (the per-thread scratch is sized for that), else at the largest of 32, 64 and 128
+   (the largest block it accepts) that keeps every scene resident, 64 at least for scenes of more
+   than 32 bodies on average. Results are the same bits under every configuration. */
 typedef struct {
   uint32_t block_threads;
   uint32_t smem_budget;
@@ -145,8 +146,8 @@ int steel_autotune(steel_batch* b, uint32_t frames, steel_tiles* best, float* be
    waits: STEEL_E_TIMEOUT, never a hang); the prepare's scan-based passes (contact classification,
    unit scan, sleep islands, coloring) stay on the team's first block.
    0: one block (the batched path). STEEL_TEAM_AUTO, the default: a scene of at least 2048 bodies or
-   64 articulations gets one thread per body or a warp per articulation, capped by the blocks that
-   fit the GPU. Other values: that many blocks (STEEL_E_INVALID if more than fit). Team launches
+   64 articulations gets eight threads per body or eight warps per articulation, capped by the blocks
+   that fit the GPU. Other values: that many blocks (STEEL_E_INVALID if more than fit). Team launches
    run the 512-thread kernel instances (one block per SM): under tiles of another block size, and
    for batches of several scenes or scenes with Nesterov momentum, the batch runs one block per
    scene. Results are the same bits either way. steel_get_team returns the blocks in use (0: one block). */

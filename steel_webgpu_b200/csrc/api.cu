@@ -459,7 +459,9 @@ uint32_t stage_flags(const SceneDev& d, uint32_t budget, uint64_t body_cap) {
 // Blocks of the team launches of prepare and solve (team.cuh) for the batch's block size and shared
 // memory: a batch of one scene without Nesterov momentum, on the 512-thread instances;
 // STEEL_TEAM_AUTO takes scenes of at least TEAM_MIN_BODIES bodies or TEAM_MIN_ARTS articulations,
-// with one thread per body or a warp per articulation, capped by the blocks that fit the GPU. Fewer
+// with eight threads per body or eight warps per articulation, capped by the blocks that fit the
+// GPU (a color's rows and the articulations spread over that many SMs: 128 quadrupeds and 8 chains
+// 7.7 ms a frame on 9 blocks, 6.1 on 72; an 8192-body pile 22.9 on 16, 21.5 on 128). Fewer
 // than two blocks: the one-block path. `strict`: a request for more blocks than fit, or under
 // smaller tiles, is an error (steel_set_team) rather than capped (a later change of tiles).
 int team_blocks_for(const steel_batch* b, uint32_t req, bool strict, uint32_t* out) {
@@ -477,7 +479,7 @@ int team_blocks_for(const steel_batch* b, uint32_t req, bool strict, uint32_t* o
   const uint32_t cap = per_sm > 0 ? (uint32_t)per_sm * (uint32_t)b->ctx->sms : 0u;
   uint32_t n = 0u;
   if (req == STEEL_TEAM_AUTO) {
-    if (d.NB >= TEAM_MIN_BODIES || d.NA >= TEAM_MIN_ARTS) n = std::min((std::max(d.NB, 32u * d.NA) + T - 1u) / T, cap);
+    if (d.NB >= TEAM_MIN_BODIES || d.NA >= TEAM_MIN_ARTS) n = std::min(8u * ((std::max(d.NB, 32u * d.NA) + T - 1u) / T), cap);
   } else {
     if (req > cap && strict)
       return fail(STEEL_E_INVALID, "at most " + std::to_string(cap) + " team blocks of " + std::to_string(T) +
@@ -634,7 +636,7 @@ int apply_tiles(steel_batch* b, const steel_tiles& t) {
   if (t.stream_groups > 8u) return fail(STEEL_E_INVALID, "at most 8 stream groups");
   const uint32_t n = (uint32_t)b->sc.size();
   std::vector<uint32_t> stages(n);
-  size_t prep = 0, solve = 0, team = 0;
+  size_t prep = 0, solve = 0, team = 0, rows = 0;
   // Dynamic shared memory a solve block may use without lowering the blocks per SM that this batch
   // can keep resident (a batch of no more scenes than SMs: one block with all of it). What the
   // scene's staging leaves holds its packed rows, so the solve reads them at shared-memory latency.
@@ -653,7 +655,8 @@ int apply_tiles(steel_batch* b, const steel_tiles& t) {
     // to the articulated passes that way than by reserving the capacity MAXC.
     const uint32_t free_bodies = d.NB - std::min(d.NB, d.NL);
     const size_t tiles = free_bodies + d.NL / 4u + std::min(d.NCOL, free_bodies) + 2u;
-    solve = std::max(solve, std::max(staged, std::min(room, staged + 128u + tiles * PK_TILE)));
+    solve = std::max(solve, staged);
+    rows = std::max(rows, staged + 128u + tiles * PK_TILE);
     // The coloring's row lists, 8 bytes a row, for 12 rows per free body and 2 per link. Larger scenes
     // keep the memory as L1: reserving 100-200 KB that their rows then overflow made a 700-body
     // pile's prepare 1.74 ms against 1.59 ms, and an 8192-body pile's 2.33 against 1.64.
@@ -662,6 +665,10 @@ int apply_tiles(steel_batch* b, const steel_tiles& t) {
     if (lists > 64u * 1024u) lists = 0u;
     prep = std::max(prep, std::max(prep_staged, std::min(prep_room, prep_staged + lists)));
   }
+  // Only when the largest scene's estimate fits: shared memory that rows then overflow is missing as
+  // L1 (a 700-body pile 26.9 ms a frame with 222 KB reserved, 23.2 without; 256 uneven scenes 20.4
+  // and 18.4).
+  if (rows <= room) solve = std::max(solve, rows);
   CU(cudaSetDevice(b->ctx->device));
   cudaStream_t st = b->ctx->stream;
   CU(cudaStreamSynchronize(st));
@@ -686,6 +693,20 @@ int apply_tiles(steel_batch* b, const steel_tiles& t) {
   b->tile_cfg.stream_groups = b->groups.empty() ? 1u : (uint32_t)b->groups.size();
   drop_graph(b);
   return update_team(b);
+}
+
+// Block size a batch starts with: 512 for no more scenes than SMs. For more, the largest of 32, 64 and
+// 128 that keeps all of them resident at once (a second wave of blocks costs as much as the first:
+// 1024 quadrupeds 5.9 ms a frame on 128 threads, 4.6 on 64; 1500 arms 1.35 and, on 32, 0.68), but 64
+// at least for scenes of more than 32 bodies on average, whose parallel passes need the threads.
+uint32_t default_threads(const steel_batch* b) {
+  if (b->max_threads == (uint32_t)BIG_THREADS) return b->max_threads;
+  const uint64_t n = b->sc.size();
+  uint64_t bodies = 0;
+  for (auto& s : b->sc) bodies += s.d.NB;
+  uint32_t t = DEFAULT_THREADS;
+  while (t > 32u && n > (uint64_t)b->ctx->sms * blocks_per_sm_of(t)) t /= 2u;
+  return std::max<uint32_t>(t, bodies > 32u * n ? 64u : 32u);
 }
 
 SceneHost* scene_of(steel_batch* b, uint32_t s) { return (b && s < b->sc.size()) ? &b->sc[s] : nullptr; }
@@ -879,7 +900,7 @@ int steel_batch_create(steel_ctx* ctx, const steel_scene_desc* scenes, uint32_t 
   CU(configure_sort(b->sort_keys));
   {
     steel_tiles t{};
-    t.block_threads = b->max_threads;  // one block per SM for few scenes, 4 per SM otherwise
+    t.block_threads = default_threads(b.get());
     t.smem_budget = 0;                 // the per-part staging caps alone
     t.narrow_blocks_per_sm = 0;        // as many as fit
     t.stream_groups = 1;               // one launch sequence

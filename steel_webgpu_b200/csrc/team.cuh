@@ -40,7 +40,12 @@ template <> struct Team<true> {
   uint32_t* error;  // the batch's device error word
   uint32_t limit;   // polls of the counter per barrier before giving up
   uint32_t* state;  // this block's shared words: [0] barriers passed, [1] nonzero after a timeout
-  __device__ uint32_t rank() const { return blockIdx.x * blockDim.x + threadIdx.x; }
+  // Consecutive warps of the team are on consecutive blocks, so a loop over a few thousand rows or
+  // bodies, or over the articulations, spreads over all SMs (a color of 1,200 rows took three of 148
+  // blocks when ranks ran through a block first).
+  __device__ uint32_t rank() const {
+    return ((threadIdx.x >> 5u) * gridDim.x + blockIdx.x) * 32u + (threadIdx.x & 31u);
+  }
   __device__ uint32_t size() const { return gridDim.x * blockDim.x; }
   __device__ bool lead() const { return blockIdx.x == 0u && threadIdx.x == 0u; }
   __device__ void sync() const {
