@@ -362,7 +362,7 @@ struct SolverT {
   }
   // A free body's spin and rolling rows of contact row `row` under normal load nl2.
   // Twists go in and out by value, so the caller's stay in registers.
-  struct Twists { f3 ta0, ta1, tb0, tb1; };
+  struct Twists { f3 ta0, ta1, tb0, tb1; bool impulse; };
   // (`sv` too: a call through the object's address would keep it in local memory.)
   static __device__ __noinline__ Twists free_angular(const SolverT sv, uint32_t row, int a, int b, f3 n, f3 t1, f3 t2, float nl2, f3 ta0, f3 ta1,
                                               f3 tb0, f3 tb1) {
@@ -388,7 +388,7 @@ struct SolverT {
     const f3 tq = (n * ds + t1 * d1) + t2 * d2;
     sv.add_imp(a, sp3(0.0f), -tq);
     sv.add_imp(b, sp3(0.0f), tq);
-    return Twists{ta[0], ta[1], tb[0], tb[1]};
+    return Twists{ta[0], ta[1], tb[0], tb[1], !(ns == 0.0f && lr.x == 0.0f && lr.y == 0.0f)};
   }
   // EXT compiles the articulated angular block in (the solve kernel's EXT instance, launched for
   // batches with a scene that has it or the contact-then-internal schedule); the EXT = false kernel
@@ -550,9 +550,10 @@ struct SolverT {
     PKF_UNIT = 32u,                 // its impulse counts in the load of its unit of several rows
     PKF_POOL = 64u,                 // its friction bound is the unit's pooled load (patch anchor)
     PKF_FINITE = 128u,              // a zero impulse times its responses is zero, not NaN
-    PKF_ANG = 256u                  // it carries the free bodies' spin and rolling rows
+    PKF_ANG = 256u,                 // it carries the free bodies' spin and rolling rows
+    PKF_ANZ = 512u                  // and they have an impulse
   };
-  static constexpr uint32_t PKF_SHIFT = 23u;  // row index below, flags above
+  static constexpr uint32_t PKF_SHIFT = 22u;  // row index below, flags above
   char* pk;              // packed rows: PK_TILE bytes per tile (shared or global)
   const uint32_t* pkc;   // team launches with rows in shared memory: this block's first chunk of each color
   __device__ bool packed() const {
@@ -628,6 +629,11 @@ struct SolverT {
       fin += ((la.x * 0.0f + la.y * 0.0f) + la.z * 0.0f) + ((aa.x * 0.0f + aa.y * 0.0f) + aa.z * 0.0f);
       fin += ((lb.x * 0.0f + lb.y * 0.0f) + lb.z * 0.0f) + ((ab.x * 0.0f + ab.y * 0.0f) + ab.z * 0.0f);
     }
+    if ((fl & PKF_ANG) != 0u)  // their responses and blocks too
+      for (uint32_t k = 19u; k < 34u; k++) {
+        const float4 v = R[k];
+        fin += ((v.x * 0.0f + v.y * 0.0f) + v.z * 0.0f);
+      }
     if (fin == 0.0f) fl |= PKF_FINITE;
     pf(p, 0) = r0;
     pf(p, 1) = mf4(v3(r3), r1.w);
@@ -716,7 +722,10 @@ struct SolverT {
       const bool flat = (__float_as_uint(lam.y) | __float_as_uint(lam.z)) == 0u;
       lam.x = nl;
       if ((fl & PKF_POOL) != 0u) lam.w = lim;
-      if (same && (flat || !(fric || it < S.FSTART)) && (!fric || lim <= 0.0f) && (fl & (PKF_FINITE | (ANG ? PKF_ANG : 0u))) == PKF_FINITE &&
+      // Spin and rolling rows without impulse under a zero load change nothing either (they would set
+      // their zero impulses' signs, which only a -0 twist could tell, and no sum makes a new one).
+      const bool ang_idle = !ANG || (fl & PKF_ANG) == 0u || ((fl & PKF_ANZ) == 0u && pooled == 0.0f);
+      if (same && (flat || !(fric || it < S.FSTART)) && (!fric || lim <= 0.0f) && (fl & PKF_FINITE) != 0u && ang_idle &&
           !minus_zero(ta0, ta1) && !minus_zero(tb0, tb1)) {
         if (__float_as_uint(lam.w) != __float_as_uint(h.f3.w)) pf(p, 3) = lam;
         return;
@@ -792,6 +801,7 @@ struct SolverT {
     if (ANG && (fl & PKF_ANG) != 0u) {
       const Twists r = free_angular(*this, row, a, b, n, t1, t2, pooled, ta0, ta1, tb0, tb1);
       ta0 = r.ta0; ta1 = r.ta1; tb0 = r.tb0; tb1 = r.tb1;
+      if (r.impulse != ((fl & PKF_ANZ) != 0u)) pf(p, 4).y = __uint_as_float(rf ^ (PKF_ANZ << PKF_SHIFT));
     }
     if (a >= 0) { tw[2 * a] = mf4(ta0, 0.0f); tw[2 * a + 1] = mf4(ta1, 0.0f); }
     if (b >= 0) { tw[2 * b] = mf4(tb0, 0.0f); tw[2 * b + 1] = mf4(tb1, 0.0f); }
