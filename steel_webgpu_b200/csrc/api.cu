@@ -441,15 +441,15 @@ void drop_graph(steel_batch* b) {
 // Shared-memory staging flags of a scene under a per-block budget of dynamic shared memory (0: the
 // per-part caps alone). Link blocks first, then twists and impulses, qd, and the color masks; a part
 // is staged when it is under its cap and both kernels' layouts stay within the budget.
-// body_cap: the cap on twists and impulses.
-uint32_t stage_flags(const SceneDev& d, uint32_t budget, uint64_t body_cap) {
+// body_cap, link_cap: the caps on twists and impulses and on link blocks.
+uint32_t stage_flags(const SceneDev& d, uint32_t budget, uint64_t body_cap, uint64_t link_cap) {
   const uint64_t lim = budget ? budget : ~0ull;
   auto fits = [&](uint32_t f) {
     return prep_smem_layout(f, d.NL, d.NB, d.NCOLW, d.NCOL).total <= lim &&
            solve_smem_layout(f, d.NB, d.ND, d.NCOL, d.NL).total <= lim;
   };
   uint32_t st = 0u;
-  if (d.NL > 0u && 4ull * d.NL * 268u <= STAGE_LINK_CAP && fits(st | STAGE_LINKS)) st |= STAGE_LINKS;
+  if (d.NL > 0u && 4ull * d.NL * 268u <= link_cap && fits(st | STAGE_LINKS)) st |= STAGE_LINKS;
   if (64ull * d.NB <= body_cap && fits(st | STAGE_BODIES)) st |= STAGE_BODIES;
   if (4ull * d.ND <= STAGE_QD_CAP && fits(st | STAGE_QD)) st |= STAGE_QD;
   if (4ull * d.NB * d.NCOLW <= STAGE_WMASK_CAP && fits(st | STAGE_WMASK)) st |= STAGE_WMASK;
@@ -644,10 +644,11 @@ int apply_tiles(steel_batch* b, const steel_tiles& t) {
                                                (n + (uint32_t)b->ctx->sms - 1u) / (uint32_t)b->ctx->sms);
   const size_t room = std::min<size_t>(t.smem_budget ? t.smem_budget : SMEM_PER_SM, solve_smem_room(resident));
   const size_t prep_room = std::min<size_t>(t.smem_budget ? t.smem_budget : SMEM_PER_SM, prep_smem_room(resident));
+  const uint64_t link_cap = n > (uint32_t)b->ctx->sms ? STAGE_LINK_CAP_MANY : STAGE_LINK_CAP;
   const uint64_t body_cap = std::max<uint64_t>(STAGE_BODY_CAP, room / 3u);
   for (uint32_t i = 0; i < n; i++) {
     SceneDev& d = b->sc[i].d;
-    d.stage = stage_flags(d, t.smem_budget, body_cap);
+    d.stage = stage_flags(d, t.smem_budget, body_cap, link_cap);
     stages[i] = d.stage;
     team = std::max<size_t>(team, solve_smem_layout(0u, d.NB, d.ND, d.NCOL, d.NL).total);
     const size_t staged = solve_smem_layout(d.stage, d.NB, d.ND, d.NCOL, d.NL).total;

@@ -110,8 +110,9 @@ struct RadixDev {
 // fits the cap; the launch's dynamic shared memory is the largest staged scene's need.
 enum : uint32_t { STAGE_LINKS = 1u, STAGE_BODIES = 2u, STAGE_QD = 4u, STAGE_WMASK = 8u };
 // Caps keep four prepare / solve blocks resident per SM.
-constexpr uint32_t STAGE_LINK_CAP = 16u * 1024u;   // link blocks (NL * 1072 B): a quadruped's, not a 40-link chain's (43 KB,
-                                                   // which serve better as L1: 64 served instances 5.2 -> 4.2 ms a frame)
+constexpr uint32_t STAGE_LINK_CAP = 44u * 1024u;   // link blocks (NL * 1072 B), batches of no more scenes than SMs
+constexpr uint32_t STAGE_LINK_CAP_MANY = 16u * 1024u;  // larger batches: a quadruped's, not a 40-link chain's (43 KB, which
+                                                       // serve better as L1: served instances 5.2 -> 4.2 ms a frame)
 constexpr uint32_t STAGE_BODY_CAP = 8u * 1024u;    // twists + impulses (NB * 64 B)
 constexpr uint32_t STAGE_QD_CAP = 8u * 1024u;      // generalized velocities of the solve (ND * 4 B)
 constexpr uint32_t STAGE_WMASK_CAP = 16u * 1024u;  // per-body color masks (NB * NCOLW words)
