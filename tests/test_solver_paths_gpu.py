@@ -77,3 +77,23 @@ def test_packed_rows(boxes, tiles, steel, oracle_lib):
         b.add_shape_box(body, hx=0.1, hy=0.1, hz=0.1, mu=0.6)
     scene = b.finalize()
     _same_as_oracle(pack(scene, caps=CAPS), oracle_lib, 15, tiles)
+
+
+@pytest.mark.parametrize("spin", [1e-18, 1e-21, 1e-24, 1e-30, 1e-42])
+@pytest.mark.parametrize("linked", [False, True])
+def test_unloaded_spin_and_rolling_rows(spin, linked, steel, oracle_lib):
+    """Contacts that are near but carry no load, between bodies that turn so slowly that the square of
+    the rolling impulse underflows: its length is 0, so the bound 0 does not clip it and it applies."""
+    b = SceneBuilder(fps=240)
+    b.add_ground_plane(mu=0.6)
+    for i, (x, y, z) in enumerate(((1.0, 2.0, 0.0), (-3.0, 0.5, 4.0), (0.0, 0.0, 1.0), (-0.0, 7.0, 0.0))):
+        body = b.add_body(xform=[0.5 * i, 0.0, 0.1, 0, 0, 0, 1], twist=[0.0, 0.0, 0.0, spin * x, spin * y, spin * z])
+        b.add_shape_sphere(body, radius=0.08, mu=0.6)
+        if linked:
+            b.add_joint_free(body)
+            tail = b.add_body(xform=[0.5 * i + 0.2, 0.0, 0.1, 0, 0, 0, 1])
+            b.add_shape_sphere(tail, radius=0.06, mu=0.6)
+            b.add_joint_revolute(body, tail, axis=[0, 1, 0], parent_xform=[0.1, 0, 0, 0, 0, 0, 1],
+                                 child_xform=[-0.1, 0, 0, 0, 0, 0, 1])
+    scene = b.finalize(solver=dict(free_rigid_torsional_friction=0.05, free_rigid_rolling_friction=0.01))
+    _same_as_oracle(pack(scene, caps=CAPS), oracle_lib, 2)
