@@ -199,7 +199,8 @@ int steel_read_contacts(steel_batch* b, uint32_t scene, float* records, uint32_t
    solve kernel (ending the frame after the last substep). steel_read_words copies
    `count` 4-byte words from one of a scene's device buffers ("art", "rows", "sched", "slots", "warm",
    "contacts") at a word offset; steel_layout_get returns a named offset of that layout (an A_* or
-   S_* offset, or ROWS). */
+   S_* offset, or ROWS), or the dynamic shared memory of the batch's prepare or solve launches
+   ("prep_smem", "solve_smem"). */
 int steel_debug_stage(steel_batch* b, int stage);
 int steel_read_words(steel_batch* b, uint32_t scene, const char* buffer, uint64_t offset, uint64_t count, void* out);
 int steel_layout_get(steel_batch* b, uint32_t scene, const char* key, uint64_t* value);

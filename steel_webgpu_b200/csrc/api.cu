@@ -652,18 +652,20 @@ int apply_tiles(steel_batch* b, const steel_tiles& t) {
     stages[i] = d.stage;
     team = std::max<size_t>(team, solve_smem_layout(0u, d.NB, d.ND, d.NCOL, d.NL).total);
     const size_t staged = solve_smem_layout(d.stage, d.NB, d.ND, d.NCOL, d.NL).total;
-    // Room for 8 rows per free body and 2 per link, a partly filled tile per color; more L1 is left
-    // to the articulated passes that way than by reserving the capacity MAXC.
+    // Room for 8 rows per free body, a partly filled tile per color; more L1 is left to the articulated
+    // passes that way than by reserving the capacity MAXC. A scene of articulations alone takes none: its
+    // few contact rows gain less than its dense rows and link blocks lose as L1 (2 rows a link: 1024
+    // quadrupeds 5.21 ms a frame, without 4.92; a 65-link chain 19.9, without 14.4).
     const uint32_t free_bodies = d.NB - std::min(d.NB, d.NL);
-    const size_t tiles = free_bodies + d.NL / 4u + std::min(d.NCOL, free_bodies) + 2u;
+    const size_t tiles = free_bodies + std::min(d.NCOL, free_bodies) + 2u;
     solve = std::max(solve, staged);
-    rows = std::max(rows, staged + 128u + tiles * PK_TILE);
+    if (rows_packed(d) && free_bodies > 0u) rows = std::max(rows, staged + 128u + tiles * PK_TILE);
     // The coloring's row lists, 8 bytes a row, for 12 rows per free body and 2 per link. Larger scenes
     // keep the memory as L1: reserving 100-200 KB that their rows then overflow made a 700-body
     // pile's prepare 1.74 ms against 1.59 ms, and an 8192-body pile's 2.33 against 1.64.
     const size_t prep_staged = prep_smem_layout(d.stage, d.NL, d.NB, d.NCOLW, d.NCOL).total;
     size_t lists = 8u * (12u * (size_t)free_bodies + 2u * d.NL) + 8u * (size_t)d.NB + 64u;
-    if (lists > 64u * 1024u) lists = 0u;
+    if (lists > 64u * 1024u || d.LONGEST_FIRST != 0u) lists = 0u;
     prep = std::max(prep, std::max(prep_staged, std::min(prep_room, prep_staged + lists)));
   }
   // Only when the largest scene's estimate fits: shared memory that rows then overflow is missing as
@@ -1547,6 +1549,9 @@ int steel_layout_get(steel_batch* b, uint32_t scene, const char* key, uint64_t* 
   L1(S_UKEY) L1(S_USIZE) L1(S_USTART) L1(S_RUNIT) L1(S_RCON) L1(S_PCOL) L1(S_PORD) L1(S_CSTART) L1(S_META)
   L1(S_KEEP) L1(S_CORDER) L1(S_KEPT)
 #undef L1
+  // Dynamic shared memory of the batch's prepare and solve launches, in bytes.
+  if (!std::strcmp(key, "prep_smem")) { *value = b->bd.prep_smem; return STEEL_OK; }
+  if (!std::strcmp(key, "solve_smem")) { *value = b->bd.solve_smem; return STEEL_OK; }
   return fail(STEEL_E_INVALID, std::string("unknown layout key ") + key);
 }
 

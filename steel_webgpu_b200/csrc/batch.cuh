@@ -97,6 +97,13 @@ constexpr uint32_t COLOR_WAIT_LIMIT = 1u << 22;  // passes of a thread over its 
 // slices for TEAM_SCRATCH_BLOCKS blocks, so the prepare's scratch passes spread over that many.
 constexpr uint32_t TEAM_MIN_BODIES = 2048u, TEAM_MIN_ARTS = 64u, TEAM_SCRATCH_BLOCKS = 32u;
 constexpr uint32_t PK_TILE = 15u * 128u;  // bytes of a tile of 8 packed solver rows: 15 float4 fields (solve.cuh)
+constexpr uint32_t PK_ROW_BITS = 22u;       // bits of a packed row's index
+// Whether a scene's contact rows are packed for the solve. Scenes with the coupled friction modes,
+// articulated torsion or cone friction, compliance, momentum or a velocity pass keep the row records.
+SHD bool rows_packed(const SceneDev& d) {
+  return d.FMODE == 0u && d.ANG_ART == 0u && d.TORS == 0u && d.NEST == 0u && d.COMPL == 0u && d.VELITERS == 0u &&
+         d.MAXC <= (1u << PK_ROW_BITS);
+}
 struct RadixDev {
   uint4* keys[2];     // ping-pong key buffers [MAXC] (x pair, y feature, z hash, w raw index)
   uint32_t* status;   // [RS_DIGITS][tiles][256] look-back words: bits 30-31 flag (1 tile count, 2 prefix)

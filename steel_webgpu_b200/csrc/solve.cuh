@@ -541,8 +541,7 @@ struct SolverT {
   // eigenvector, the anchor bias) is computed here with the operations the visit would use.
   // About 70% of the visits are of contacts that are near but not touching and change nothing: such
   // a visit stops after the normal impulse, having read the first five fields.
-  // Scenes with the coupled friction modes, articulated torsion or cone friction, compliance,
-  // momentum or a velocity pass keep the row records (solve_row).
+  // Scenes that rows_packed leaves out keep the row records (solve_row).
   enum : uint32_t {
     PKF_LA = 1u, PKF_LB = 2u,       // the side is a link (linear response in the row record)
     PKF_IA = 4u, PKF_IB = 8u,       // the side collects link impulses (kind 2)
@@ -553,13 +552,10 @@ struct SolverT {
     PKF_ANG = 256u,                 // it carries the free bodies' spin and rolling rows
     PKF_ANZ = 512u                  // and they have an impulse
   };
-  static constexpr uint32_t PKF_SHIFT = 22u;  // row index below, flags above
+  static constexpr uint32_t PKF_SHIFT = PK_ROW_BITS;  // row index below, flags above
   char* pk;              // packed rows: PK_TILE bytes per tile (shared or global)
   const uint32_t* pkc;   // team launches with rows in shared memory: this block's first chunk of each color
-  __device__ bool packed() const {
-    return S.FMODE == 0u && S.ANG_ART == 0u && S.TORS == 0u && S.NEST == 0u && S.COMPL == 0u && S.VELITERS == 0u &&
-           S.MAXC <= (1u << PKF_SHIFT);
-  }
+  __device__ bool packed() const { return rows_packed(S); }
   // Address of row i of color c in the global layout: color c's tiles start at (its first slot) / 8
   // + c, which leaves each color room for its partly filled last tile.
   static __device__ size_t pk_offset(const uint32_t* wcs, uint32_t c, uint32_t i) {

@@ -97,3 +97,42 @@ def test_unloaded_spin_and_rolling_rows(spin, linked, steel, oracle_lib):
                                  child_xform=[-0.1, 0, 0, 0, 0, 0, 1])
     scene = b.finalize(solver=dict(free_rigid_torsional_friction=0.05, free_rigid_rolling_friction=0.01))
     _same_as_oracle(pack(scene, caps=CAPS), oracle_lib, 2)
+
+
+PACKED_TILE = 15 * 128  # bytes of 8 packed rows
+UNPACKED = {"coupled": ({}, {"friction_mode": "bisection"}), "momentum": (dict(nesterov_momentum=True), None),
+            "compliance": (dict(contact_compliance=True, enable_restitution=False), None),
+            "velocity": (dict(velocity_iterations=4), None)}
+
+
+def _boxes(n, solver):
+    b = SceneBuilder(fps=240, box_hulls="direct")
+    b.add_ground_plane(mu=0.6)
+    for i in range(n):
+        body = b.add_body(xform=[0.25 * i, 0.0, 0.101, 0, 0, 0, 1])
+        b.add_shape_box(body, hx=0.1, hy=0.1, hz=0.1, mu=0.6)
+    return b.finalize(solver=solver)
+
+
+@pytest.mark.parametrize("name", ["plain", "chain", "longest_first"] + list(UNPACKED))
+def test_shared_memory_of_rows_that_are_not_there(name, steel):
+    """The solve reserves shared memory for packed rows of free bodies alone, the prepare for row
+    lists where the coloring makes them: what is reserved and not used is missing as L1."""
+    solver, opts = UNPACKED.get(name, ({}, None))
+    if name == "longest_first":
+        opts = {"propagation_color_order": "longest_first"}
+    scene = _chains(10, 0.0) if name == "chain" else _boxes(40, solver)
+    pk = pack(scene, opts={"solver": opts} if opts else None, caps=CAPS)
+    g = Batch([pk])
+    solve, prep = g.layout("solve_smem"), g.layout("prep_smem")
+    g.close()
+    link = 268 * 4  # staged per link in both kernels; twists and impulses 64 B a body, qd 4 B a dof in the solve
+    staged = link * (pk.NB if name == "chain" else 0)
+    if name in ("plain", "longest_first"):
+        assert solve > staged + 40 * PACKED_TILE
+    else:
+        assert solve <= staged + 68 * pk.NB + 1024
+    if name == "longest_first":
+        assert prep <= staged + 4 * 2 * pk.NB + 1024  # color counts and masks
+    elif name == "plain":
+        assert prep > staged + 8 * 12 * 40
