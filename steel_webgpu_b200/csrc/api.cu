@@ -808,7 +808,7 @@ int steel_batch_create(steel_ctx* ctx, const steel_scene_desc* scenes, uint32_t 
   CU(cudaMemsetAsync(b->arena, 0, b->arena_bytes, st));
   uint8_t* A = b->arena;
   std::vector<SceneDev> dev(n);
-  uint32_t art_f64 = 0, solve_ext = 0;
+  uint32_t art_f64 = 0, solve_ext = 0, solve_rows = 0;
   for (uint32_t i = 0; i < n; i++) {
     SceneHost& s = b->sc[i];
     SceneDev& d = s.d;
@@ -846,6 +846,7 @@ int steel_batch_create(steel_ctx* ctx, const steel_scene_desc* scenes, uint32_t 
     d.stage = 0u;  // set by apply_tiles below
     art_f64 |= d.ART_F64;
     solve_ext |= d.ANG_ART | d.CTI;
+    solve_rows |= rows_packed(d) ? ROWS_PACKED : ROWS_RECORDS;
     dev[i] = d;
     CU(cudaMemcpyAsync((void*)d.sf.p, s.statF.data(), s.statF.size() * 4, cudaMemcpyHostToDevice, st));
     CU(cudaMemcpyAsync((void*)d.lt.p, s.levels.data(), s.levels.size() * 4, cudaMemcpyHostToDevice, st));
@@ -888,6 +889,7 @@ int steel_batch_create(steel_ctx* ctx, const steel_scene_desc* scenes, uint32_t 
   bd.team_blocks = 0;
   bd.art_f64 = art_f64 != 0u ? 1u : 0u;
   bd.solve_ext = solve_ext != 0u ? 1u : 0u;
+  bd.solve_rows = solve_rows;
   bd.block_threads = b->max_threads;
   bd.wait_limit = STEEL_WAIT_LIMIT_DEFAULT;
   bd.trace_prep = nullptr;

@@ -30,6 +30,7 @@ struct BatchDev {
   uint32_t team_smem;         // dynamic shared memory of k_solve_team launches (nothing staged)
   uint32_t art_f64;           // some scene has ART_F64: launch the prepare instances that carry it
   uint32_t solve_ext;         // some scene has ANG_ART or CTI: launch the solve instances that carry them
+  uint32_t solve_rows;        // ROWS_*: whether the scenes' contact rows are packed, launch the instance for that
   uint32_t block_threads;     // threads per prepare / solve block (one of BLOCK_SIZES)
   uint32_t wait_limit;        // try_wait rounds of a shared-memory bulk copy (BULK_WAIT_LIMIT unless a test
                               // lowers it to make the bounded wait run out)
@@ -97,6 +98,7 @@ constexpr uint32_t COLOR_WAIT_LIMIT = 1u << 22;  // passes of a thread over its 
 // slices for TEAM_SCRATCH_BLOCKS blocks, so the prepare's scratch passes spread over that many.
 constexpr uint32_t TEAM_MIN_BODIES = 2048u, TEAM_MIN_ARTS = 64u, TEAM_SCRATCH_BLOCKS = 32u;
 constexpr uint32_t PK_TILE = 15u * 128u;  // bytes of a tile of 8 packed solver rows: 15 float4 fields (solve.cuh)
+enum : uint32_t { ROWS_PACKED = 1u, ROWS_RECORDS = 2u, ROWS_BOTH = 3u };
 constexpr uint32_t PK_ROW_BITS = 22u;       // bits of a packed row's index
 // Whether a scene's contact rows are packed for the solve. Scenes with the coupled friction modes,
 // articulated torsion or cone friction, compliance, momentum or a velocity pass keep the row records.

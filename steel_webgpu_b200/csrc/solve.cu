@@ -15,39 +15,57 @@ namespace steel {
 namespace STEEL_NS {
 // EXT: the batch has a scene with torsional/rolling friction of articulated contacts or the
 // contact-then-internal row schedule; only that instance carries the 5-row angular block in its
-// contact loop and the two-phase iteration.
-template <bool EXT>
+// contact loop and the two-phase iteration. ROWS: which of the solve's bodies the instance has, by what
+// the batch's scenes need (solve_scene).
+template <bool EXT, uint32_t ROWS>
 __global__ void __launch_bounds__(STEEL_BLOCK, blocks_per_sm_of(STEEL_BLOCK)) k_solve(BatchDev B) {
   const uint32_t sc = B.order[blockIdx.x];
   const unsigned long long t0 = B.trace_solve ? trace_clock() : 0ull;
-  solve_scene<EXT, false>(B, sc, Team<false>{});
+  solve_scene<EXT, false, ROWS>(B, sc, Team<false>{});
   if (B.trace_solve) trace_block(B.trace_solve + 3ull * sc, t0);
 }
 #if STEEL_BLOCK == 512  // team launches run the 512-thread instances (one block per SM)
 // A batch of one large scene: every block of this cooperative launch solves it together (team.cuh).
-template <bool EXT>
+template <bool EXT, uint32_t ROWS>
 __global__ void __launch_bounds__(STEEL_BLOCK, blocks_per_sm_of(STEEL_BLOCK)) k_solve_team(BatchDev B) {
   __shared__ uint32_t team_state[2];
   if (threadIdx.x == 0u) { team_state[0] = 0u; team_state[1] = 0u; }  // published by copy_scene's barrier
   const uint32_t sc = B.order[0];
   const unsigned long long t0 = B.trace_solve ? trace_clock() : 0ull;
-  solve_scene<EXT, true>(B, sc, Team<true>{B.team_bar, B.error, TEAM_WAIT_LIMIT, team_state});
+  solve_scene<EXT, true, ROWS>(B, sc, Team<true>{B.team_bar, B.error, TEAM_WAIT_LIMIT, team_state});
   if (B.trace_solve && blockIdx.x == 0u) trace_block(B.trace_solve + 3ull * sc, t0);
 }
 #endif
 }  // namespace STEEL_NS
 
+typedef void (*SolveKernel)(BatchDev);
+// The instance for a batch: [EXT][ROWS_*], and the team's (a batch of one scene is never mixed).
+static SolveKernel solve_kernel(bool ext, uint32_t rows) {
+  static const SolveKernel k[2][3] = {
+      {STEEL_NS::k_solve<false, ROWS_PACKED>, STEEL_NS::k_solve<false, ROWS_RECORDS>, STEEL_NS::k_solve<false, ROWS_BOTH>},
+      {STEEL_NS::k_solve<true, ROWS_PACKED>, STEEL_NS::k_solve<true, ROWS_RECORDS>, STEEL_NS::k_solve<true, ROWS_BOTH>}};
+  return k[ext ? 1 : 0][rows - ROWS_PACKED];
+}
+#if STEEL_BLOCK == 512
+static SolveKernel solve_team_kernel(bool ext, uint32_t rows) {
+  if (rows == ROWS_PACKED) return ext ? STEEL_NS::k_solve_team<true, ROWS_PACKED> : STEEL_NS::k_solve_team<false, ROWS_PACKED>;
+  return ext ? STEEL_NS::k_solve_team<true, ROWS_RECORDS> : STEEL_NS::k_solve_team<false, ROWS_RECORDS>;
+}
+#endif
+
 template <>
 cudaError_t configure_solve_t<STEEL_BLOCK>(size_t smem_bytes) {
-  const void* fns[] = {(const void*)STEEL_NS::k_solve<false>, (const void*)STEEL_NS::k_solve<true>,
+  for (uint32_t ext = 0; ext < 2u; ext++)
+    for (uint32_t rows = ROWS_PACKED; rows <= ROWS_BOTH; rows++) {
+      cudaError_t e = cudaFuncSetAttribute((const void*)solve_kernel(ext != 0u, rows),
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
 #if STEEL_BLOCK == 512
-                       (const void*)STEEL_NS::k_solve_team<false>, (const void*)STEEL_NS::k_solve_team<true>
+      if (e == cudaSuccess && rows != ROWS_BOTH)
+        e = cudaFuncSetAttribute((const void*)solve_team_kernel(ext != 0u, rows),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
 #endif
-  };
-  for (const void* f : fns) {
-    cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-    if (e != cudaSuccess) return e;
-  }
+      if (e != cudaSuccess) return e;
+    }
   return cudaSuccess;
 }
 template <>
@@ -65,8 +83,7 @@ void launch_solve_t<STEEL_BLOCK>(const BatchDev& b, cudaStream_t st) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     cudaMemsetAsync(b.team_bar, 0, sizeof(uint32_t), st);
-    if (b.solve_ext) cudaLaunchKernelEx(&cfg, STEEL_NS::k_solve_team<true>, b);
-    else cudaLaunchKernelEx(&cfg, STEEL_NS::k_solve_team<false>, b);
+    cudaLaunchKernelEx(&cfg, solve_team_kernel(b.solve_ext != 0u, b.solve_rows), b);
     return;
   }
 #endif
@@ -83,17 +100,19 @@ void launch_solve_t<STEEL_BLOCK>(const BatchDev& b, cudaStream_t st) {
   at[0].val.sharedMemCarveout = solve_carveout(b);
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if (b.solve_ext) cudaLaunchKernelEx(&cfg, STEEL_NS::k_solve<true>, b);
-  else cudaLaunchKernelEx(&cfg, STEEL_NS::k_solve<false>, b);
+  cudaLaunchKernelEx(&cfg, solve_kernel(b.solve_ext != 0u, b.solve_rows), b);
 }
 template <>
 int solve_team_blocks_per_sm_t<STEEL_BLOCK>(size_t smem_bytes) {
 #if STEEL_BLOCK == 512
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, STEEL_NS::k_solve_team<true>, STEEL_BLOCK, smem_bytes) !=
-      cudaSuccess)
-    return 0;
-  return n;
+  int least = 0;
+  for (uint32_t k = 0; k < 4u; k++) {
+    int n = 0;
+    const SolveKernel f = solve_team_kernel((k & 1u) != 0u, (k & 2u) != 0u ? ROWS_RECORDS : ROWS_PACKED);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, STEEL_BLOCK, smem_bytes) != cudaSuccess) return 0;
+    if (k == 0u || n < least) least = n;
+  }
+  return least;
 #else
   (void)smem_bytes;
   return 0;

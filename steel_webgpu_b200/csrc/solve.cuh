@@ -512,14 +512,14 @@ struct SolverT {
     if (a >= 0) { tw[(uint32_t)a * 2u] = mf4(ta[0], 0.0f); tw[(uint32_t)a * 2u + 1u] = mf4(ta[1], 0.0f); }
     if (b >= 0) { tw[(uint32_t)b * 2u] = mf4(tb[0], 0.0f); tw[(uint32_t)b * 2u + 1u] = mf4(tb[1], 0.0f); }
   }
-  // The EXT contact loop is a function (by value, as free_angular), so its cone code's frame and
-  // registers stay out of the solve loop.
+  // The EXT row is a function (by value, as free_angular), so its cone code's frame and registers stay
+  // out of the solve loop.
   static __device__ __noinline__ void solve_row_ext(const SolverT sv, uint32_t us, uint32_t row, int a, int b,
                                                     uint32_t mode, uint32_t it) {
     sv.template solve_row<true>(us, row, a, b, mode, it);
   }
   template <bool EXT>
-  __device__ void solve_slot(uint32_t u, uint32_t mode, uint32_t it) const {
+  __device__ __forceinline__ void solve_slot(uint32_t u, uint32_t mode, uint32_t it) const {
     float4 sl = S.slots[2u * u];
     if (EXT) solve_row_ext(*this, f2u(sl.y), f2u(sl.x), f2i(sl.z), f2i(sl.w), mode, it);
     else solve_row<EXT>(f2u(sl.y), f2u(sl.x), f2i(sl.z), f2i(sl.w), mode, it);
@@ -555,7 +555,6 @@ struct SolverT {
   static constexpr uint32_t PKF_SHIFT = PK_ROW_BITS;  // row index below, flags above
   char* pk;              // packed rows: PK_TILE bytes per tile (shared or global)
   const uint32_t* pkc;   // team launches with rows in shared memory: this block's first chunk of each color
-  __device__ bool packed() const { return rows_packed(S); }
   // Address of row i of color c in the global layout: color c's tiles start at (its first slot) / 8
   // + c, which leaves each color room for its partly filled last tile.
   static __device__ size_t pk_offset(const uint32_t* wcs, uint32_t c, uint32_t i) {
@@ -1426,8 +1425,8 @@ struct SolverT {
     }
     __syncthreads();
   }
-  // One sweep (wgsl.js:3559-3611).
-  template <bool EXT>
+  // One sweep (wgsl.js:3559-3611). PACKED: the contact rows are packed.
+  template <bool EXT, bool PACKED>
   // Inline: a separate function's calling convention spilled the packed rows' registers (568 bytes).
   // ph: 0 every row; 1 contacts only (no joint-internal rows, no velocity-limit rows, no internal
   // dense rows); 2 joint-internal rows only (no contact slots, no contact dense rows). The two
@@ -1435,7 +1434,7 @@ struct SolverT {
   __device__ __forceinline__ void sweep(uint32_t mode, uint32_t ncol0, uint32_t it, const uint32_t* wcs, uint32_t nu, uint32_t ph) const {
     const uint32_t tid = tm.rank(), nt = tm.size();
     const uint32_t ncol = ph == 2u ? 0u : ncol0;
-    const bool pk_on = packed();
+    constexpr bool pk_on = PACKED;
     const uint32_t lane = threadIdx.x & 31u;  // a warp per articulation
     if (ph != 1u)
       for (uint32_t a = tid >> 5u; a < S.NA; a += nt >> 5u) joint_rows(a, lane);
@@ -1542,16 +1541,18 @@ struct SolverT {
 // stages nothing in shared memory: twists, impulses, qd and link blocks stay in global memory,
 // where every block sees them after a grid barrier. Each block keeps its own copy of the scene
 // descriptor, the parameters and the color starts.
-template <bool EXT, bool TEAM>
-__device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team<TEAM> tm) {
+struct SolveShared {
+  Params params;
+  SceneDev scene;  // the scene's offsets and sizes, read everywhere in the serial passes
+  uint64_t stage_bar;
+  uint32_t scan[33];
+};
+template <bool EXT, bool TEAM, bool PACKED>
+__device__ __forceinline__ void solve_rows(const BatchDev& B, SolveShared& sh, Team<TEAM> tm) {
   extern __shared__ float4 ssm4[];  // solve_smem_layout: [tw | imp], qd, color starts, link blocks
-  __shared__ Params Ps;
-  __shared__ SceneDev Ss;  // the scene's offsets and sizes, read everywhere in the serial passes
   const uint32_t tid = tm.rank(), nt = tm.size();
-  if (B.active[sc] == 0u) return;  // not stepping in this frame (serving loop)
-  copy_scene(Ss, B.scenes[sc]);
-  const SceneDev& S = Ss;
-  if (threadIdx.x == 0u) Ps = *S.params;
+  const SceneDev& S = sh.scene;
+  if (threadIdx.x == 0u) sh.params = *S.params;
   uint8_t* sb = reinterpret_cast<uint8_t*>(ssm4);
   const uint32_t stage = TEAM ? 0u : S.stage;
   const SolveSmem lay = solve_smem_layout(stage, S.NB, S.ND, S.NCOL, S.NL);
@@ -1562,13 +1563,12 @@ __device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team
   const uint32_t ncol = min(S.sched[S.S_META + 1u], S.NCOL);
   for (uint32_t i = threadIdx.x; i < S.NCOL + 2u; i += blockDim.x) wcs[i] = S.sched[S.S_CSTART + i];
   // Link blocks into shared memory with one bulk copy (A_LINK is 16-byte aligned).
-  __shared__ __align__(8) uint64_t stage_bar;
-  if (staged_links && !stage_to_shared(lb, S.art + S.A_LINK, 4u * S.NL * LBLK, &stage_bar, B.wait_limit)) {
+  if (staged_links && !stage_to_shared(lb, S.art + S.A_LINK, 4u * S.NL * LBLK, &sh.stage_bar, B.wait_limit)) {
     if (threadIdx.x == 0u) atomicCAS(B.error, 0u, (uint32_t)ERR_STAGE_TIMEOUT);
     return;  // the whole block: the result above is the same in every thread
   }
   __syncthreads();
-  const Params& P = Ps;
+  const Params& P = sh.params;
   SolverT<TEAM> sv(tm, S, P, lb, staged_bodies ? reinterpret_cast<float4*>(sb + lay.tw) : S.tw,
                    staged_bodies ? reinterpret_cast<float4*>(sb + lay.imp) : S.imp,
                    (stage & STAGE_QD) ? reinterpret_cast<float*>(sb + lay.aqd) : S.aqd);
@@ -1617,7 +1617,7 @@ __device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team
   for (uint32_t i = tid; i < 2u * S.ND; i += nt) A[S.A_LIM + i] = 0.0f;
   for (uint32_t i = tid; i < S.ND; i += nt) { A[S.A_FRIC + i] = 0.0f; A[S.A_DRV + i] = 0.0f; }
   const uint32_t nslot = wcs[S.NCOL + 1u];
-  const bool pk_on = sv.packed();
+  constexpr bool pk_on = PACKED;
   // Packed rows in shared memory when they fit what the launch has beyond the scene's staging: the
   // whole scene's, or in a team launch this block's chunks (copied from the global layout below).
   char* pk_global = reinterpret_cast<char*>(S.pk);
@@ -1652,12 +1652,9 @@ __device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team
     for (uint32_t a = tid; a < S.NA; a += nt) sv.ar.twists(a, sv.aqd, sv.tw);
   }
   tm.sync();
-  {
-    // The dense lists are built by one block (the whole team's block 0), then published.
-    __shared__ uint32_t dtmp[33];
-    if (!TEAM || blockIdx.x == 0u) sv.dense_lists(dtmp);
-    if (TEAM) tm.sync();
-  }
+  // The dense lists are built by one block (the whole team's block 0), then published.
+  if (!TEAM || blockIdx.x == 0u) sv.dense_lists(sh.scan);
+  if (TEAM) tm.sync();
   // Velocity pass (velocity_iterations, wgsl.js:3700-3736): positions integrate with the velocities
   // reached here; further bias-free sweeps from the accumulated impulses set the output velocities.
   auto velocity_snapshot = [&]() {
@@ -1702,10 +1699,10 @@ __device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team
   // contact iterations (phase 1), then the joint-internal rows (phase 2); otherwise one pass of full
   // sweeps (phase 0). Only the EXT instance carries it.
   const bool cti = EXT && S.CTI == 1u;
-  const uint32_t npos = (cti ? 2u : 1u) * P.iterations;
-  for (uint32_t k = 0; k <= npos + S.VELITERS; k++) {
+  const uint32_t npos = (cti ? 2u : 1u) * P.iterations, nvel = PACKED ? 0u : S.VELITERS;
+  for (uint32_t k = 0; k <= npos + nvel; k++) {
     uint32_t it = 0u, ph = 0u;
-    if (k > npos) {
+    if (!PACKED && k > npos) {
       if (k == npos + 1u) velocity_snapshot();
       it = P.iterations + (k - npos - 1u);
     } else if (k > 0u) {
@@ -1713,9 +1710,9 @@ __device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team
       it = k - 1u - (second ? P.iterations : 0u);
       if (cti) ph = second ? 2u : 1u;
       // Nesterov momentum keeps block-wide sums: a team launch is never made for a scene with it.
-      if (!TEAM && S.NEST == 1u && !second) sv.momentum_step(ncol, it, wcs);
+      if (!TEAM && !PACKED && S.NEST == 1u && !second) sv.momentum_step(ncol, it, wcs);
     }
-    sv.template sweep<EXT>(k == 0u ? 0u : 1u, ncol, it, wcs, nu, ph);
+    sv.template sweep<EXT, PACKED>(k == 0u ? 0u : 1u, ncol, it, wcs, nu, ph);
   }
   sv.vpass = false;
   if (pk_on) {
@@ -1765,7 +1762,7 @@ __device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team
     float damp = (sv.bflags((int)b) & 1u) != 0u ? 1.0f : 1.0f - S.sf[S.SF_BODY + b * 8u + 3u].w * P.dt;
     S.lv[b] = mf4(v, 0.0f);
     S.av[b] = mf4(w * damp, 0.0f);
-    if (S.VELITERS > 0u) {
+    if (!PACKED && S.VELITERS > 0u) {
       f3 s2[2];
       sv.snap_tw((int)b, s2);
       v = s2[0];
@@ -1784,7 +1781,7 @@ __device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team
   }
   for (uint32_t i = tid; i < S.ND; i += nt) {
     A[S.A_QD + i] = sv.aqd[i];
-    if (S.VELITERS > 0u) sv.aqd[i] = A[S.A_SNAP + S.NB * 8u + i];
+    if (!PACKED && S.VELITERS > 0u) sv.aqd[i] = A[S.A_SNAP + S.NB * 8u + i];
   }
   tm.sync();
   for (uint32_t l = tid; l < S.NL; l += nt) {
@@ -1861,7 +1858,7 @@ __device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team
       f3 ta[2], tb[2];
       sv.load_tw(a, ta);
       sv.load_tw(b, tb);
-      if (S.VELITERS > 0u) { sv.snap_tw(a, ta); sv.snap_tw(b, tb); }
+      if (!PACKED && S.VELITERS > 0u) { sv.snap_tw(a, ta); sv.snap_tw(b, tb); }
       f3 vrel = (tb[0] + cross(tb[1], frb)) - (ta[0] + cross(ta[1], fra));
       float4 lam = rows[o + 6u];
       f3 lt = t1 * lam.y + t2 * lam.z;
@@ -1910,6 +1907,20 @@ __device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team
     tm.sync();
     for (uint32_t i = tid; i < S.NL * LBLK; i += nt) S.art[S.A_LINK + i] = lb[i];
   }
+}
+
+// The solve of packed rows and that of row records (rows_packed) are compiled apart, each inline, so
+// that neither's registers and frame weigh on the other, and an instance has the one that its batch
+// needs (ROWS; both for a mixed batch). With the record rows beside the packed ones in one sweep, 60
+// stacked boxes took 23.5 ms a frame with coupled friction, 19.0 with momentum and 22.6 with a velocity
+// pass; apart 20.3, 16.2 and 19.9.
+template <bool EXT, bool TEAM, uint32_t ROWS>
+__device__ __forceinline__ void solve_scene(const BatchDev& B, uint32_t sc, Team<TEAM> tm) {
+  __shared__ SolveShared sh;
+  if (B.active[sc] == 0u) return;  // not stepping in this frame (serving loop)
+  copy_scene(sh.scene, B.scenes[sc]);
+  if (ROWS == ROWS_PACKED || (ROWS == ROWS_BOTH && rows_packed(sh.scene))) solve_rows<EXT, TEAM, true>(B, sh, tm);
+  else solve_rows<EXT, TEAM, false>(B, sh, tm);
 }
 
 }  // namespace steel

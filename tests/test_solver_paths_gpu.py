@@ -136,3 +136,26 @@ def test_shared_memory_of_rows_that_are_not_there(name, steel):
         assert prep <= staged + 4 * 2 * pk.NB + 1024  # color counts and masks
     elif name == "plain":
         assert prep > staged + 8 * 12 * 40
+
+
+@pytest.mark.parametrize("tiles", [(), (32,), (512,)])
+@pytest.mark.parametrize("ext", [False, True])
+def test_batch_of_packed_and_record_rows(tiles, ext, steel, oracle_lib):
+    """A batch whose scenes need both solve bodies, and each scene in a batch of its own kind."""
+    kinds = [({}, {"row_schedule": "contact_then_internal"} if ext else None)] + list(UNPACKED.values()) + [({}, None)]
+    pks = [pack(_boxes(5 + i, solver), opts={"solver": opts} if opts else None) for i, (solver, opts) in enumerate(kinds)]
+    g = Batch(pks)
+    if tiles:
+        g.set_tiles(*tiles)
+    g.step(12)
+    for i, pk in enumerate(pks):
+        o = oracle_lib.OracleSim(pk)
+        o.step(12)
+        alone = Batch([pk])
+        alone.step(12)
+        for batch, scene in ((g, i), (alone, 0)):
+            pose, vel = batch.raw_state(scene)[:2]
+            assert np.array_equal(_bits(o.read("poses")[:pk.NB * 8]), _bits(pose)), i
+            assert np.array_equal(_bits(o.read("vel")[:pk.NB * 8]), _bits(vel)), i
+        alone.close()
+    g.close()
