@@ -189,6 +189,7 @@ void build_levels(SceneHost& s) {
     const int p = parent(l);
     depth[l] = p >= 0 && (uint32_t)p < l ? depth[p] + 1u : 0u;
   }
+  d.ART_LINKS = d.ART_LEVELS = 0u;
   for (uint32_t a = 0; a < NA; a++) {
     const uint32_t* ai = s.statU.data() + d.SU_ART + a * 4u;
     uint32_t top = 0u;
@@ -199,6 +200,8 @@ void build_levels(SceneHost& s) {
       lvo.push_back((uint32_t)lvl.size());
     }
     lvb[a + 1u] = (uint32_t)lvo.size() - 1u;
+    d.ART_LINKS = std::max(d.ART_LINKS, ai[1]);
+    d.ART_LEVELS = std::max(d.ART_LEVELS, top);
   }
   std::vector<std::vector<uint32_t>> children(NL);
   for (uint32_t l = NL; l-- > 0u;)

@@ -1262,19 +1262,20 @@ struct Art {
       }
     }
   }
-  // Propagation of the link impulses L_P and joint impulses L_TAU of articulation a by one warp (all
-  // 32 lanes call it; every lane's earlier writes to them are visible after a __syncwarp). Links of
-  // one tree level are independent, so a quadruped takes 4 steps rather than 13: toward the root a
+  // Propagation of the link impulses L_P and joint impulses L_TAU of articulation a by one warp (step
+  // 32: all lanes call it, every lane's earlier writes to them visible after a __syncwarp) or by one
+  // thread (lane 0, step 1). Links of one tree level are independent, so a quadruped takes a warp 4
+  // steps rather than 13: toward the root a
   // link adds its children's contributions (kept in their L_DV) in the order the serial pass meets
   // them, last child first; from the root each link reads its parent's L_DV. One thread per
   // articulation took 68,000 cycles on a quadruped.
   // (`ar` by value: a call through the object's address would keep it in local memory.)
-  static __device__ __noinline__ void apply_warp(const Art ar, uint32_t a, float* aqd, float4* tw, uint32_t lane) {
+  static __device__ __noinline__ void apply(const Art ar, uint32_t a, float* aqd, float4* tw, uint32_t lane, uint32_t step) {
     const uint32_t r0 = ar.S.lt[a], r1 = ar.S.lt[a + 1u];
     RO<uint32_t> lvo = ar.S.lt + ar.S.LT_LVO, lvl = ar.S.lt + ar.S.LT_LVL, chs = ar.S.lt + ar.S.LT_CHS, chl = ar.S.lt + ar.S.LT_CHL;
     for (uint32_t k = r1; k-- > r0;) {
       const uint32_t e = lvo[k + 1u];
-      for (uint32_t i = lvo[k] + lane; i < e; i += 32u) {
+      for (uint32_t i = lvo[k] + lane; i < e; i += step) {
         const uint32_t l = lvl[i], L = ar.lo(l), n = ar.lndof(l);
         const uint32_t c1 = chs[l + 1u];
         SVec p = ar.ldsv(L + L_P);
@@ -1310,11 +1311,11 @@ struct Art {
         }
         ar.stsv(L + L_DV, fshift(p, ar.link_r(l)));
       }
-      __syncwarp();
+      if (step > 1u) __syncwarp();
     }
     for (uint32_t k = r0; k < r1; k++) {
       const uint32_t e = lvo[k + 1u];
-      for (uint32_t i = lvo[k] + lane; i < e; i += 32u) {
+      for (uint32_t i = lvo[k] + lane; i < e; i += step) {
         const uint32_t l = lvl[i], L = ar.lo(l), n = ar.lndof(l), d0 = ar.ldof(l);
         const int par = ar.lparent(l);
         SVec dv = sv0();
@@ -1342,7 +1343,7 @@ struct Art {
         ar.stsv(L + L_P, sv0());
         for (uint32_t r = 0; r < ar.JMc; r++) ar.LB[L + L_TAU + r] = 0.0f;
       }
-      __syncwarp();
+      if (step > 1u) __syncwarp();
     }
   }
 };

@@ -235,6 +235,7 @@ struct SceneDev {
   // lt[LT_CHL + lt[LT_CHS + l] ...).
   RO<uint32_t> lt;
   uint32_t LT_LVO, LT_LVL, LT_CHS, LT_CHL;
+  uint32_t ART_LINKS, ART_LEVELS;    // the most links and levels of one articulation
   float4* bpc;                       // prepare: contact reduction values (plane position, gap, identity) [MAXC]
   float* tscr;                       // per-thread scratch slices (path temporaries), TSCR floats each
   uint32_t TSCR;

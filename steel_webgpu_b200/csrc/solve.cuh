@@ -1195,18 +1195,43 @@ struct SolverT {
   // so only its own joint and dense rows move it. FRESH: its link twists are those of its qd (set by a
   // twist pass, cleared by apply). QUIET: every dense row was idle at its present qd.
   enum : uint32_t { AS_ALONE = 1u, AS_FRESH = 2u, AS_QUIET = 4u };
-  __device__ void art_apply(uint32_t a, uint32_t lane) const {
-    __syncwarp();
-    Art::apply_warp(ar, a, aqd, tw, lane);
-    if (lane == 0u) S.sched[S.S_DSTATE + a] &= AS_ALONE;
-    __syncwarp();
+  // The joint and impulse passes take a warp or a thread per articulation. Both are chains of dependent
+  // link steps: a warp takes a tree level a step and the articulations of its turn one after another,
+  // a thread a link a step, all at once. So a warp each while there are warps for all, or while their
+  // turns' levels are no more than the links (threads up to 32 apart, as the team allows, so that few
+  // share a warp). A frame by warps and by threads: 200 bodies of two links in a 512-thread block 11.1
+  // and 5.7 ms, 60 flaps of one link 1.90 and 1.41, 60 quadrupeds 9.6 and 9.9 (their solve after landing
+  // 1.71 and 1.53 ms); 24 quadrupeds, by warps, 4.9, by neighboring threads 7.8.
+  uint32_t art_shift = 5u;  // log2 of the threads from one articulation's first to the next one's
+  bool art_warp = true;
+  __device__ void art_split() {
+    const uint32_t nt = tm.size(), nw = nt >> 5u;
+    art_warp = S.NA <= nw || (S.NA + nw - 1u) / nw * S.ART_LEVELS <= (S.NA + nt - 1u) / nt * S.ART_LINKS;
+    if (!art_warp)
+      for (art_shift = 0u; art_shift < 5u && S.NA <= nt >> (art_shift + 1u);) art_shift++;
   }
-  // Exact articulation update from the contact impulses on its links (wgsl.js:3380-3394), by a warp.
+  // f(a, lane) for this thread's articulations: by all lanes of a warp, or by one thread as lane 0.
+  template <class F>
+  __device__ __forceinline__ void each_articulation(const F& f) const {
+    const uint32_t tid = tm.rank(), lane = tid & ((1u << art_shift) - 1u);
+    if (!art_warp && lane != 0u) return;
+    for (uint32_t a = tid >> art_shift; a < S.NA; a += tm.size() >> art_shift) f(a, lane);
+  }
+  __device__ void art_sync() const {
+    if (art_warp) __syncwarp();
+  }
+  __device__ void art_apply(uint32_t a, uint32_t lane) const {
+    art_sync();
+    Art::apply(ar, a, aqd, tw, lane, art_warp ? 32u : 1u);
+    if (lane == 0u) S.sched[S.S_DSTATE + a] &= AS_ALONE;
+    art_sync();
+  }
+  // Exact articulation update from the contact impulses on its links (wgsl.js:3380-3394).
   __device__ void contact_impulses(uint32_t a, uint32_t lane) const {
     if ((S.sched[S.S_DSTATE + a] & AS_ALONE) != 0u) return;
     uint4 ai = ar.info(a);
     bool hit = false;
-    for (uint32_t k = lane; k < ai.y; k += 32u) {
+    for (uint32_t k = lane; k < ai.y; k += art_warp ? 32u : 1u) {
       uint32_t l = ai.x + k;
       uint32_t b = (uint32_t)ar.lbody(l);
       f3 f = v3(imp[b * 2u]), t = v3(imp[b * 2u + 1u]);
@@ -1217,20 +1242,21 @@ struct SolverT {
         imp[b * 2u + 1u] = make_float4(0, 0, 0, 0);
       }
     }
-    if (__any_sync(0xffffffffu, hit)) art_apply(a, lane);
+    if (art_warp) hit = __any_sync(0xffffffffu, hit);
+    if (hit) art_apply(a, lane);
   }
-  // One joint impulse: every lane has computed it; lane 0 stores, the warp propagates it.
+  // One joint impulse: every lane has computed it; lane 0 stores, all propagate it.
   __device__ void joint_impulse(uint32_t a, uint32_t l, uint32_t r, float* slot, float value, float tau,
                                 uint32_t lane) const {
-    __syncwarp();  // every lane has read what lane 0 overwrites
+    art_sync();  // every lane has read what lane 0 overwrites
     if (lane == 0u) {
       if (slot != nullptr) *slot = value;
       ar.LB[ar.lo(l) + L_TAU + r] = tau;
     }
     art_apply(a, lane);
   }
-  // Joint friction and limit rows over the dofs listed in prepare (wgsl.js:3404-3468), by a warp: the
-  // lanes compute each row alike (one after another, as each moves qd) and share its propagation.
+  // Joint friction and limit rows over the dofs listed in prepare (wgsl.js:3404-3468): the lanes compute
+  // each row alike (one after another, as each moves qd) and share its propagation.
   __device__ void joint_rows(uint32_t a, uint32_t lane) const {
     float* A = S.art;
     uint32_t n = f2u(A[S.A_RLN + a]);
@@ -1280,7 +1306,7 @@ struct SolverT {
     }
   }
   // Joint velocity limits after the contact impulses (wgsl.js:3413-3419, 3462-3467): a stateless
-  // push back onto |qd| <= limit for the marked dofs of revolute, prismatic and D6 links. By a warp.
+  // push back onto |qd| <= limit for the marked dofs of revolute, prismatic and D6 links.
   __device__ void vlim_rows(uint32_t a, uint32_t lane) const {
     float* A = S.art;
     if (A[S.A_AVL + a] <= 0.5f) return;
@@ -1419,10 +1445,10 @@ struct SolverT {
         momentum_unit(S.sched[S.S_RUNIT + row], row, beta, it == 0u);
       }
     __syncthreads();
-    for (uint32_t a = tid >> 5u; a < S.NA; a += nt >> 5u) {
-      contact_impulses(a, tid & 31u);
-      if (S.VLIM_ON == 1u) vlim_rows(a, tid & 31u);
-    }
+    each_articulation([&](uint32_t a, uint32_t lane) {
+      contact_impulses(a, lane);
+      if (S.VLIM_ON == 1u) vlim_rows(a, lane);
+    });
     __syncthreads();
   }
   // One sweep (wgsl.js:3559-3611). PACKED: the contact rows are packed.
@@ -1435,9 +1461,8 @@ struct SolverT {
     const uint32_t tid = tm.rank(), nt = tm.size();
     const uint32_t ncol = ph == 2u ? 0u : ncol0;
     constexpr bool pk_on = PACKED;
-    const uint32_t lane = threadIdx.x & 31u;  // a warp per articulation
     if (ph != 1u)
-      for (uint32_t a = tid >> 5u; a < S.NA; a += nt >> 5u) joint_rows(a, lane);
+      each_articulation([&](uint32_t a, uint32_t lane) { joint_rows(a, lane); });
     if (S.PATCH == 1u && mode == 1u) {
       // Four units per thread at a time, their loads issued together (each unit's sum keeps its
       // row order).
@@ -1483,10 +1508,10 @@ struct SolverT {
         for (uint32_t u = wcs[S.NCOL]; u < wcs[S.NCOL + 1u]; u++) solve_slot<EXT>(u, mode, it);
     }
     tm.sync();
-    for (uint32_t a = tid >> 5u; a < S.NA; a += nt >> 5u) {
+    each_articulation([&](uint32_t a, uint32_t lane) {
       contact_impulses(a, lane);
       if (S.VLIM_ON == 1u && ph != 1u) vlim_rows(a, lane);
-    }
+    });
     tm.sync();
     if (S.VLIM_FREE == 1u) {
       for (uint32_t b = tid; b < S.NB; b += nt) {
@@ -1572,6 +1597,7 @@ __device__ __forceinline__ void solve_rows(const BatchDev& B, SolveShared& sh, T
   SolverT<TEAM> sv(tm, S, P, lb, staged_bodies ? reinterpret_cast<float4*>(sb + lay.tw) : S.tw,
                    staged_bodies ? reinterpret_cast<float4*>(sb + lay.imp) : S.imp,
                    (stage & STAGE_QD) ? reinterpret_cast<float*>(sb + lay.aqd) : S.aqd);
+  sv.art_split();
   float* A = S.art;
   // Prologue (wgsl.js:3635-3691).
   for (uint32_t i = tid; i < S.ND; i += nt) sv.aqd[i] = A[S.A_QDH + i];

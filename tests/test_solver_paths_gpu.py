@@ -159,3 +159,32 @@ def test_batch_of_packed_and_record_rows(tiles, ext, steel, oracle_lib):
             assert np.array_equal(_bits(o.read("vel")[:pk.NB * 8]), _bits(vel)), i
         alone.close()
     g.close()
+
+
+@pytest.mark.parametrize("kind,count", [("flap", 1), ("flap", 17), ("flap", 33), ("floater", 2), ("floater", 5),
+                                        ("floater", 33), ("quadruped", 1), ("quadruped", 3), ("quadruped", 4)])
+@pytest.mark.parametrize("threads", [32, 64, 512])
+def test_articulations_by_warps_and_by_threads(kind, count, threads, steel, oracle_lib):
+    """Joint and impulse passes at the edges of the split: as many articulations as warps, more (by
+    threads, 32 down to 1 apart), and more than threads; with contacts, limits and joint friction."""
+    rng = np.random.default_rng(count)
+    b = SceneBuilder(fps=240, box_hulls="direct")
+    b.add_ground_plane(mu=0.6)
+    for i in range(count):
+        x, y = 1.2 * (i % 6), 1.2 * (i // 6)
+        joint = dict(limitLower=-0.2, limitUpper=0.1, friction=0.05, velocityLimit=2.0)
+        if kind == "quadruped":
+            synth._add_quadruped(b, rng, [x, y, 0.7])
+            continue
+        base, z, at = -1, 0.05, [x - 0.1, y, 0.05]
+        if kind == "floater":
+            base = b.add_body(xform=[x - 0.2, y, 0.06, 0, 0, 0, 1], twist=[0.1, 0.0, 0.0, 0.0, 0.0, 1.0])
+            b.add_shape_box(base, hx=0.1, hy=0.1, hz=0.05, mu=0.6)
+            b.add_joint_free(base)
+            at = [0.1, 0.0, -0.01]
+        flap = b.add_body(xform=[x, y, z, 0, 0, 0, 1])
+        b.add_shape_box(flap, hx=0.09, hy=0.1, hz=0.02, mu=0.6)
+        b.add_joint_revolute(base, flap, axis=[0, 1, 0], parent_xform=at + [0, 0, 0, 1],
+                             child_xform=[-0.1, 0, 0, 0, 0, 0, 1], q=[0.05 * (i % 3)], **joint)
+    scene = b.finalize(solver=dict(enable_joint_friction=True, enable_joint_velocity_limits=True))
+    _same_as_oracle(pack(scene, caps=CAPS), oracle_lib, 10, (threads,))
