@@ -926,9 +926,10 @@ __device__ __forceinline__ void prepare_scene(const BatchDev& B, uint32_t sc, Te
     if (F64 && S.ART_F64 == 1u) ar.factor<true>(a, P);
     else ar.factor<false>(a, P);
   };
-  if (S.NA <= 4u * (nt >> 5u)) {
-    // Few articulations: a warp each, lanes over links and matrix elements. Beyond four to a warp a
-    // thread each has more of them in flight.
+  if (S.NA <= 3u * (nt >> 5u)) {
+    // Few articulations: a warp each, lanes over links and matrix elements. Beyond three to a warp a
+    // thread each has more of them in flight (a prepare by warps and by threads: two quadrupeds a warp
+    // 0.49 and 0.56 ms, three 0.66 and 0.66, four 0.99 and 0.92; four swinging flaps a warp 60 and 30 us).
     const uint32_t lane = tid & 31u;
     for (uint32_t a = tid >> 5u; a < S.NA; a += nt >> 5u) {
       gate(a, lane, 32u);

@@ -188,3 +188,22 @@ def test_articulations_by_warps_and_by_threads(kind, count, threads, steel, orac
                              child_xform=[-0.1, 0, 0, 0, 0, 0, 1], q=[0.05 * (i % 3)], **joint)
     scene = b.finalize(solver=dict(enable_joint_friction=True, enable_joint_velocity_limits=True))
     _same_as_oracle(pack(scene, caps=CAPS), oracle_lib, 10, (threads,))
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+@pytest.mark.parametrize("count", [3, 4, 7])
+def test_factorisation_by_warps_and_by_threads(fp64, count, steel, oracle_lib):
+    """Articulated inertias of trees with a floating base at the split's edge: three to the one warp of
+    a 32-thread block, four (by threads), and both by the warps of a 512-thread block."""
+    rng = np.random.default_rng(count)
+    b = SceneBuilder(fps=240, box_hulls="direct")
+    b.add_ground_plane(mu=0.7)
+    for i in range(count):
+        if i % 2 == 0:
+            synth._add_quadruped(b, rng, [1.2 * i, 0.0, 0.75])
+        else:
+            synth._add_chain(b, rng, [1.2 * i, 0.0, 1.6], 9, ratio_max=1000.0)
+    scene = b.finalize()
+    pk = pack(scene, opts={"solver": {"articulation_fp64": True}} if fp64 else None, caps=CAPS)
+    _same_as_oracle(pk, oracle_lib, 8, (32,))
+    _same_as_oracle(pk, oracle_lib, 8, (512,))
