@@ -554,18 +554,10 @@ struct SolverT {
   };
   static constexpr uint32_t PKF_SHIFT = PK_ROW_BITS;  // row index below, flags above
   char* pk;              // packed rows: PK_TILE bytes per tile (shared or global)
-  const uint32_t* pkc;   // team launches with rows in shared memory: this block's first chunk of each color
   // Address of row i of color c in the global layout: color c's tiles start at (its first slot) / 8
   // + c, which leaves each color room for its partly filled last tile.
   static __device__ size_t pk_offset(const uint32_t* wcs, uint32_t c, uint32_t i) {
     return (size_t)((wcs[c] >> 3u) + c + (i >> 3u)) * PK_TILE + (i & 7u) * 16u;
-  }
-  // In a team launch a block keeps its own chunks of 32 rows (chunk j of a color belongs to block
-  // j mod grid, Team<true>::rank), color after color.
-  __device__ char* pk_at(const uint32_t* wcs, uint32_t c, uint32_t i) const {
-    if (TEAM && pkc != nullptr)
-      return pk + (size_t)(pkc[c] + (i >> 5u) / gridDim.x) * (4u * PK_TILE) + ((i >> 3u) & 3u) * PK_TILE + (i & 7u) * 16u;
-    return pk + pk_offset(wcs, c, i);
   }
   static __device__ float4& pf(char* p, uint32_t f) { return *reinterpret_cast<float4*>(p + f * 128u); }
   __device__ void pack_row(char* p, uint32_t row, uint32_t us, uint32_t key) const {
@@ -834,13 +826,13 @@ struct SolverT {
     for (uint32_t c = 0; c < ncol; c++) {
       const uint32_t s1 = wcs[c + 1u];
       for (uint32_t i = tid; i < s1 - s0; i += nt) {
-        char* p = pk_at(wcs, c, i);
+        char* p = pk + pk_offset(wcs, c, i);
         if (!ready) h = pk_load(p);
         ready = false;
         solve_packed<WARM, ANG>(p, h, it, omega, uload);
       }
       if (c + 1u < ncol && tid < wcs[c + 2u] - s1) {
-        h = pk_load(pk_at(wcs, c + 1u, tid));
+        h = pk_load(pk + pk_offset(wcs, c + 1u, tid));
         ready = true;
       }
       s0 = s1;
@@ -1644,23 +1636,23 @@ __device__ __forceinline__ void solve_rows(const BatchDev& B, SolveShared& sh, T
   for (uint32_t i = tid; i < S.ND; i += nt) { A[S.A_FRIC + i] = 0.0f; A[S.A_DRV + i] = 0.0f; }
   const uint32_t nslot = wcs[S.NCOL + 1u];
   constexpr bool pk_on = PACKED;
-  // Packed rows in shared memory when they fit what the launch has beyond the scene's staging: the
-  // whole scene's, or in a team launch this block's chunks (copied from the global layout below).
+  // Packed rows in shared memory when they fit what the launch has beyond the scene's staging; a team
+  // launch's, which every block reads, stay in global memory.
   char* pk_global = reinterpret_cast<char*>(S.pk);
   char* rows_sm = reinterpret_cast<char*>(sb) + ((lay.total + 127u) & ~127u);
   const uint32_t rows_room = B.solve_smem > ((lay.total + 127u) & ~127u) ? B.solve_smem - ((lay.total + 127u) & ~127u) : 0u;
   const uint32_t ncs = wcs[ncol];  // rows of the colors, without the overflow color's
-  bool rows_shared = pk_on && !TEAM && ((size_t)(ncs >> 3u) + ncol + 1u) * PK_TILE <= rows_room;
+  const bool rows_shared = pk_on && !TEAM && ((size_t)(ncs >> 3u) + ncol + 1u) * PK_TILE <= rows_room;
   sv.pk = rows_shared ? rows_sm : pk_global;
-  sv.pkc = nullptr;
   for (uint32_t u = tid; u < nslot; u += nt) {
     uint32_t row = S.sched[S.S_PORD + u], us = S.sched[S.S_RUNIT + row], key = S.sched[S.S_UKEY + us];
+    // (Packed rows do not read their slots; steel_read_words does.)
     S.slots[2u * u] = make_float4((float)row, (float)us, (float)((int)(key & 0xffffu) - 1), (float)((int)(key >> 16u) - 1));
     if (pk_on) {
       const uint32_t c = S.sched[S.S_PCOL + row];
       // The overflow color stays in global memory (one thread runs it, whichever layout the colors have).
       const size_t o = SolverT<TEAM>::pk_offset(wcs, c, u - wcs[c]);
-      sv.pack_row((rows_shared && !TEAM && c < ncol ? rows_sm : pk_global) + o, row, us, key);
+      sv.pack_row((rows_shared && c < ncol ? rows_sm : pk_global) + o, row, us, key);
     }
   }
   // An articulation no contact row touches: prepare marked the bodies of the others' links.
