@@ -89,12 +89,12 @@ struct SceneHost {
   SceneDev d{};  // device pointers filled after allocation
   // arena offsets
   size_t o_sf, o_su, o_pos, o_rot, o_ppos, o_prot, o_lv, o_av, o_spos, o_srot, o_alo, o_ahi, o_art, o_cnt, o_stats,
-      o_params, o_craw, o_con, o_ckeys, o_rows, o_slots, o_pk, o_plam, o_bpc, o_warm, o_sched, o_tw, o_imp, o_aqd, o_tscr;
+      o_params, o_craw, o_con, o_ckeys, o_rows, o_slots, o_pk, o_plam, o_warm, o_sched, o_tw, o_imp, o_aqd, o_tscr;
   // Device-wide radix sort of a scene whose padded keys may exceed the block sort's shared array.
   bool large_sort = false;
   uint32_t sort_tiles = 0;
   size_t o_rkeys1 = 0, o_rstat = 0, o_rhist = 0, o_rctr = 0;
-  size_t art_floats = 0, sched_words = 0, warm_words = 0, tscr_floats = 0;
+  size_t art_floats = 0, sched_words = 0, scratch_word = 0, warm_words = 0, tscr_floats = 0;
   std::vector<float> statF;
   std::vector<uint32_t> levels;  // SceneDev::lt
   size_t o_lt = 0, o_dhd = 0;
@@ -284,19 +284,24 @@ int build_scene(SceneHost& s, const steel_scene_desc& in, Layout& L, uint32_t th
   {
     size_t so = 0;
     auto put = [&](uint32_t& field, size_t n) { field = (uint32_t)so; so += n > 0 ? n : 1; };
-    put(d.S_UNITOF, MAXC); put(d.S_DSLOT, MAXC); put(d.S_CORDER, MAXC); put(d.S_UKEY, MAXC);
-    put(d.S_USTART0, MAXC + 1); put(d.S_USIZE, MAXC); put(d.S_USTART, MAXC + 1); put(d.S_RK0, MAXC);
-    put(d.S_RK1, MAXC); put(d.S_RK2, MAXC); put(d.S_LEAD, MAXC);
-    put(d.S_KEEP, MAXC); put(d.S_KEPT, MAXC); put(d.S_ROWOF, MAXC);
+    put(d.S_CORDER, MAXC); put(d.S_UKEY, MAXC); put(d.S_USIZE, MAXC); put(d.S_USTART, MAXC + 1);
+    put(d.S_KEEP, MAXC); put(d.S_KEPT, MAXC);
     put(d.S_RUNIT, MAXC); put(d.S_RCON, MAXC); put(d.S_PCOL, MAXC); put(d.S_PORD, MAXC);
     put(d.S_CSTART, d.NCOL + 2); put(d.S_META, 8); put(d.S_WWIN, d.WH); put(d.S_WSLOT, (size_t)MAXC + d.MAXDENSE);
     put(d.S_WMASK, (size_t)NB * d.NCOLW); put(d.S_WCOUNT, d.NCOL + 2); put(d.S_LINKHIT, NB); put(d.S_JSPLIT, NL);
     put(d.S_UF, NB + NA); put(d.S_UFF, NB + NA); put(d.S_UTP, MAXC);
     put(d.S_DSTART, NA + 1); put(d.S_DOFF, NA); put(d.S_DLIST, d.MAXDENSE);
+    put(d.S_DFIN, d.MAXDENSE); put(d.S_DSTATE, NA);
+    // What the prepare alone uses comes last: the solve's packed rows and dense list start here and
+    // reach over the raw contacts, which follow (128-byte aligned, as the tiles of rows).
+    so = (so + 31) & ~(size_t)31;
+    s.scratch_word = so;
+    put(d.S_UNITOF, MAXC); put(d.S_DSLOT, MAXC); put(d.S_USTART0, MAXC + 1); put(d.S_RK0, MAXC);
+    put(d.S_RK1, MAXC); put(d.S_RK2, MAXC); put(d.S_LEAD, MAXC); put(d.S_ROWOF, MAXC);
     // parallel coloring: per-body row lists and frontiers, row keys
     put(d.S_BSTART, NB + 1); put(d.S_BPOS, NB); put(d.S_BREADY, NB); put(d.S_BLIST, 2 * (size_t)MAXC);
     put(d.S_RKEY, MAXC); put(d.S_RFLAG, MAXC); put(d.S_WL, 2 * (size_t)NB);
-    put(d.S_DFIN, d.MAXDENSE); put(d.S_DSTATE, NA);
+    so = (so + 3) & ~(size_t)3;
     s.sched_words = so;
   }
   s.warm_words = 10ull * d.WH + 30ull * d.AH;
@@ -332,7 +337,7 @@ int build_scene(SceneHost& s, const steel_scene_desc& in, Layout& L, uint32_t th
   const size_t arena0 = L.bytes;
   s.o_sf = L.take(s.statF.size() * 4);
   s.o_su = L.take(s.statU.size() * 4);
-  s.o_lt = L.take(s.levels.size() * 4); s.o_dhd = L.take((size_t)d.MAXDENSE * 32u + 32u);
+  s.o_lt = L.take(s.levels.size() * 4);
   s.o_pos = L.take((size_t)NB * 16); s.o_rot = L.take((size_t)NB * 16);
   s.o_ppos = L.take((size_t)NB * 16); s.o_prot = L.take((size_t)NB * 16);
   s.o_lv = L.take((size_t)NB * 16); s.o_av = L.take((size_t)NB * 16);
@@ -340,7 +345,20 @@ int build_scene(SceneHost& s, const steel_scene_desc& in, Layout& L, uint32_t th
   s.o_alo = L.take((size_t)NS * 16); s.o_ahi = L.take((size_t)NS * 16);
   s.o_art = L.take(s.art_floats * 4);
   s.o_cnt = L.take(64); s.o_stats = L.take(64); s.o_params = L.take(sizeof(Params));
-  s.o_craw = L.take((size_t)MAXC * 6 * 16); s.o_con = L.take((size_t)MAXC * 6 * 16);
+  // Scheduling arrays and, right behind them, the raw contacts. From the prepare's scratch on, the solve
+  // reuses them (nothing of either is read between the prepare and the next narrowphase): packed rows
+  // from the front, the dense list's entries from the end. Both fit, as a contact becomes a row or
+  // a dense row, and the rows of loops and mimics (2 a loop, 1 a mimic) are added.
+  {
+    const size_t extra = 32u * (2u * (size_t)d.NLOOP + d.NMIMIC) + 2u * PK_TILE;
+    const size_t solve = (rows_packed(d) ? (size_t)MAXC / 8u * PK_TILE : 32u * (size_t)MAXC) + extra;
+    const size_t scratch = (s.sched_words - s.scratch_word) * 4u;
+    s.o_sched = L.take(s.scratch_word * 4u + std::max(scratch + (size_t)MAXC * 6u * 16u, solve + 32u));
+    s.o_craw = s.o_sched + s.sched_words * 4u;
+    s.o_pk = s.o_sched + s.scratch_word * 4u;
+    s.o_dhd = ((L.bytes - 32u) & ~(size_t)31);
+  }
+  s.o_con = L.take((size_t)MAXC * 6 * 16);
   s.large_sort = next_pow2(MAXC) > SORT_SMEM_KEYS;
   s.o_ckeys = L.take(s.large_sort ? (size_t)MAXC * 16 : 16);
   if (s.large_sort) {
@@ -351,10 +369,8 @@ int build_scene(SceneHost& s, const steel_scene_desc& in, Layout& L, uint32_t th
     s.o_rctr = L.take(4ull * RS_DIGITS);
   }
   s.o_rows = L.take((size_t)MAXC * d.ROWS * 16); s.o_slots = L.take((size_t)MAXC * 2 * 16);
-  s.o_pk = L.take(((size_t)MAXC / 8u + d.NCOL + 8u) * PK_TILE); s.o_plam = L.take((size_t)MAXC * 4);
-  s.o_bpc = L.take((size_t)MAXC * 16);
+  s.o_plam = L.take(rows_packed(d) && d.PATCH ? (size_t)MAXC * 4 : 16);
   s.o_warm = L.take(s.warm_words * 4);
-  s.o_sched = L.take(s.sched_words * 4);
   s.o_tw = L.take((size_t)NB * 32); s.o_imp = L.take((size_t)NB * 32);
   s.o_aqd = L.take((size_t)(ND > 0 ? ND : 1) * 4);
   const bool team_sized = one_scene && (NB >= TEAM_MIN_BODIES || d.NA >= TEAM_MIN_ARTS);
@@ -830,7 +846,7 @@ int steel_batch_create(steel_ctx* ctx, const steel_scene_desc* scenes, uint32_t 
     d.craw = at<float4>(A, s.o_craw); d.con = at<float4>(A, s.o_con); d.ckeys = at<uint4>(A, s.o_ckeys);
     d.rows = at<float4>(A, s.o_rows); d.slots = at<float4>(A, s.o_slots);
     d.pk = at<char>(A, s.o_pk); d.plam = at<float>(A, s.o_plam);
-    d.bpc = at<float4>(A, s.o_bpc);
+    d.bpc = d.craw;  // the raw contacts are sorted by then
     d.warm_tab = at<uint32_t>(A, s.o_warm); d.sched = at<uint32_t>(A, s.o_sched);
     d.tw = at<float4>(A, s.o_tw); d.imp = at<float4>(A, s.o_imp); d.aqd = at<float>(A, s.o_aqd);
     d.tscr = at<float>(A, s.o_tscr);

@@ -221,7 +221,7 @@ struct SceneDev {
   uint4* ckeys;                      // sort scratch [MAXC]
   float4* rows;                      // row records [MAXC * ROWS]
   float4* slots;                     // slot table [MAXC * 2]
-  char* pk;                          // solve: rows packed by color in tiles of 8 (solve.cuh)
+  char* pk;                          // solve: rows packed in slot order, tiles of 8 (solve.cuh)
   float* plam;                       // solve: normal impulses in row order, 0 for rows outside a patch [MAXC]
   uint32_t* warm_tab;                // warm table: 10*WH + 30*AH words
   uint32_t* sched;                   // scheduling arrays, offsets below
@@ -229,7 +229,7 @@ struct SceneDev {
       S_KEEP, S_KEPT, S_ROWOF, S_RUNIT, S_RCON, S_PCOL, S_PORD, S_CSTART, S_META, S_WWIN, S_WSLOT, S_WMASK,
       S_WCOUNT, S_LINKHIT, S_JSPLIT, S_UF, S_UFF, S_UTP, S_DSTART, S_DOFF, S_DLIST, S_BSTART, S_BPOS, S_BREADY,
       S_BLIST, S_RKEY, S_RFLAG, S_WL, S_DFIN, S_DSTATE;
-  float4* dhd;                       // solve: dense rows' impulses and scalars in list order [MAXDENSE * 2]
+  float4* dhd;                       // solve: dense rows' impulses and scalars, entry k of the list at dhd - 2 k
   // Articulation trees by level (static): level records of articulation a are [lt[a], lt[a + 1]); level
   // record k's links are lt[LT_LVL + lt[LT_LVO + k] ...); the children of link l, last first, are
   // lt[LT_CHL + lt[LT_CHS + l] ...).

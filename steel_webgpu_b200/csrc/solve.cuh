@@ -529,7 +529,7 @@ struct SolverT {
   // A contact row is visited 13 times per substep by one thread, in color order. The row records
   // (23 float4 at a stride of 368 B, in contact order) make a warp's load of one field touch 32
   // lines and come in many dependent steps: a color of a single warp took 5,700 cycles on 12 boxes.
-  // So once per solve the rows are packed color by color into tiles of 8 rows, field by field (a
+  // So once per solve the rows are packed in slot order into tiles of 8 rows, field by field (a
   // field of a tile is one 128 B line, every field at a constant offset from the row's address), in
   // shared memory when the scene's rows fit, else in global memory.
   //   0 n, 1/K      1 ra, rhs      2 rb, weight   3 impulses, anchor bound (updated by every visit)
@@ -554,11 +554,8 @@ struct SolverT {
   };
   static constexpr uint32_t PKF_SHIFT = PK_ROW_BITS;  // row index below, flags above
   char* pk;              // packed rows: PK_TILE bytes per tile (shared or global)
-  // Address of row i of color c in the global layout: color c's tiles start at (its first slot) / 8
-  // + c, which leaves each color room for its partly filled last tile.
-  static __device__ size_t pk_offset(const uint32_t* wcs, uint32_t c, uint32_t i) {
-    return (size_t)((wcs[c] >> 3u) + c + (i >> 3u)) * PK_TILE + (i & 7u) * 16u;
-  }
+  // Offset of slot u's row (a color's rows are consecutive slots).
+  static __device__ size_t pk_offset(uint32_t u) { return (size_t)(u >> 3u) * PK_TILE + (u & 7u) * 16u; }
   static __device__ float4& pf(char* p, uint32_t f) { return *reinterpret_cast<float4*>(p + f * 128u); }
   __device__ void pack_row(char* p, uint32_t row, uint32_t us, uint32_t key) const {
     const float4* R = S.rows + (size_t)row * S.ROWS;
@@ -826,13 +823,13 @@ struct SolverT {
     for (uint32_t c = 0; c < ncol; c++) {
       const uint32_t s1 = wcs[c + 1u];
       for (uint32_t i = tid; i < s1 - s0; i += nt) {
-        char* p = pk + pk_offset(wcs, c, i);
+        char* p = pk + pk_offset(s0 + i);
         if (!ready) h = pk_load(p);
         ready = false;
         solve_packed<WARM, ANG>(p, h, it, omega, uload);
       }
       if (c + 1u < ncol && tid < wcs[c + 2u] - s1) {
-        h = pk_load(pk + pk_offset(wcs, c + 1u, tid));
+        h = pk_load(pk + pk_offset(s1 + tid));
         ready = true;
       }
       s0 = s1;
@@ -841,7 +838,7 @@ struct SolverT {
     const uint32_t nover = wcs[S.NCOL + 1u] - wcs[S.NCOL];
     if (tid == 0u)
       for (uint32_t i = 0; i < nover; i++) {
-        char* p = S.pk + pk_offset(wcs, S.NCOL, i);
+        char* p = S.pk + pk_offset(wcs[S.NCOL] + i);
         solve_packed<WARM, ANG>(p, pk_load(p), it, omega, uload);
       }
   }
@@ -852,6 +849,8 @@ struct SolverT {
     for (uint32_t off = 16u; off > 0u; off >>= 1u) x += __shfl_xor_sync(0xffffffffu, x, off);
     return x;
   }
+  // Entry k of the dense list (stored from the end backwards).
+  __device__ float4* dh(uint32_t k) const { return S.dhd - 2u * k; }
   // Each articulation's dense rows in slot order (S_DSTART / S_DLIST), by a stable counting sort
   // once per solve, so the dense passes walk their own rows instead of filtering all of them (the
   // order within an articulation, the one the Gauss-Seidel pass needs, is kept). All threads of
@@ -889,8 +888,8 @@ struct SolverT {
     for (uint32_t k = tid; k < nd; k += nt) {
       const uint32_t row = list[k], o = S.A_DENSE + row * S.DPS;
       const bool bil = A[o + 21u] > 0.5f;
-      S.dhd[2u * k] = make_float4(A[o + 9u], A[o + 10u], A[o + 11u], bil ? -1.0f : (S.sched[S.S_DFIN + row] != 0u ? 1.0f : 0.0f));
-      S.dhd[2u * k + 1u] = make_float4(A[o + 3u], A[o + 4u], A[o + 5u], A[o + 24u]);
+      dh(k)[0] = make_float4(A[o + 9u], A[o + 10u], A[o + 11u], bil ? -1.0f : (S.sched[S.S_DFIN + row] != 0u ? 1.0f : 0.0f));
+      dh(k)[1] = make_float4(A[o + 3u], A[o + 4u], A[o + 5u], A[o + 24u]);
     }
     __syncthreads();
   }
@@ -936,7 +935,7 @@ struct SolverT {
                                 const float (&q)[DENSE_REG], const uint32_t* dl, float4 h0) const {
     const float* A = S.art + base0 + S.DHDR;
     const uint32_t mine = lane < n ? dl[k + lane] : 0u;
-    const float4 h1 = lane < n ? S.dhd[2u * (k + lane) + 1u] : make_float4(0, 0, 0, 0);
+    const float4 h1 = lane < n ? dh(k + lane)[1] : make_float4(0, 0, 0, 0);
     float p[32];
 #pragma unroll
     for (uint32_t i = 0; i < 32u; i++) {
@@ -999,7 +998,7 @@ struct SolverT {
         // The run of rows from k that had no impulse; in the warm sweep they are done, and so are
         // bilateral rows and the rows that this phase leaves out.
         const uint32_t n = min(32u, k1 - k);
-        const float4 h0 = lane < n ? S.dhd[2u * (k + lane)] : make_float4(0, 0, 0, 0);
+        const float4 h0 = lane < n ? dh(k + lane)[0] : make_float4(0, 0, 0, 0);
         const bool bil = h0.w < 0.0f;
         const bool left_out = ph != 0u && bil == (ph == 1u);
         const bool zero = h0.w > 0.0f && (__float_as_uint(h0.x) | __float_as_uint(h0.y) | __float_as_uint(h0.z)) == 0u;
@@ -1020,10 +1019,10 @@ struct SolverT {
       for (;;) {
         const bool more = k + 1u < k1;
         const uint32_t nrow = more ? dl[k + 1u] : row;
-        const float4 nh = more ? S.dhd[2u * (k + 1u)] : make_float4(0, 0, 0, 0);
+        const float4 nh = more ? dh(k + 1u)[0] : make_float4(0, 0, 0, 0);
         DenseRow nxt;
         if (more) dense_load(base0 + nrow * DPS, lane, ai.w, nxt);
-        dense_row(cur, base0 + row * DPS, S.dhd + 2u * k, ai, mode, it, ph, lane, q);
+        dense_row(cur, base0 + row * DPS, dh(k), ai, mode, it, ph, lane, q);
         moved = true;
         k++;
         if (!more || (ahead && nh.w > 0.0f && nh.x == 0.0f && nh.y == 0.0f && nh.z == 0.0f)) break;
@@ -1642,7 +1641,7 @@ __device__ __forceinline__ void solve_rows(const BatchDev& B, SolveShared& sh, T
   char* rows_sm = reinterpret_cast<char*>(sb) + ((lay.total + 127u) & ~127u);
   const uint32_t rows_room = B.solve_smem > ((lay.total + 127u) & ~127u) ? B.solve_smem - ((lay.total + 127u) & ~127u) : 0u;
   const uint32_t ncs = wcs[ncol];  // rows of the colors, without the overflow color's
-  const bool rows_shared = pk_on && !TEAM && ((size_t)(ncs >> 3u) + ncol + 1u) * PK_TILE <= rows_room;
+  const bool rows_shared = pk_on && !TEAM && (size_t)((ncs + 7u) >> 3u) * PK_TILE <= rows_room;
   sv.pk = rows_shared ? rows_sm : pk_global;
   for (uint32_t u = tid; u < nslot; u += nt) {
     uint32_t row = S.sched[S.S_PORD + u], us = S.sched[S.S_RUNIT + row], key = S.sched[S.S_UKEY + us];
@@ -1651,7 +1650,7 @@ __device__ __forceinline__ void solve_rows(const BatchDev& B, SolveShared& sh, T
     if (pk_on) {
       const uint32_t c = S.sched[S.S_PCOL + row];
       // The overflow color stays in global memory (one thread runs it, whichever layout the colors have).
-      const size_t o = SolverT<TEAM>::pk_offset(wcs, c, u - wcs[c]);
+      const size_t o = SolverT<TEAM>::pk_offset(u);
       sv.pack_row((rows_shared && c < ncol ? rows_sm : pk_global) + o, row, us, key);
     }
   }
@@ -1736,7 +1735,7 @@ __device__ __forceinline__ void solve_rows(const BatchDev& B, SolveShared& sh, T
   if (pk_on) {
     for (uint32_t u = tid; u < nslot; u += nt) {
       const uint32_t c = S.sched[S.S_PCOL + S.sched[S.S_PORD + u]];
-      const size_t o = SolverT<TEAM>::pk_offset(wcs, c, u - wcs[c]);
+      const size_t o = SolverT<TEAM>::pk_offset(u);
       sv.unpack_row((c < ncol ? sv.pk : pk_global) + o);
     }
     tm.sync();

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from steel_webgpu_b200 import SceneBuilder, pack, synth
-from steel_webgpu_b200.sim import Batch
+from steel_webgpu_b200.sim import Batch, auto_caps
 
 pytestmark = pytest.mark.gpu
 
@@ -207,3 +207,33 @@ def test_factorisation_by_warps_and_by_threads(fp64, count, steel, oracle_lib):
     pk = pack(scene, opts={"solver": {"articulation_fp64": True}} if fp64 else None, caps=CAPS)
     _same_as_oracle(pk, oracle_lib, 8, (32,))
     _same_as_oracle(pk, oracle_lib, 8, (512,))
+
+
+def _sized(name):
+    if name == "boxes":
+        return _boxes(64, {}), None
+    if name == "coupled":
+        return _boxes(64, {}), {"solver": {"friction_mode": "bisection"}}
+    if name == "chains":
+        return _chains(40, 2.0), None
+    b = SceneBuilder(fps=240, box_hulls="direct")
+    b.add_ground_plane(mu=0.6)
+    synth._add_quadruped(b, np.random.default_rng(1), [0.0, 0.0, 0.75])
+    return b.finalize(), None
+
+
+# Device bytes of a scene with its automatic capacities, alone and in a batch of 200, before rows were packed.
+SCENE_BYTES = {"boxes": (1137664, 1033216), "coupled": (1109504, 1005056), "chains": (6647296, 2948608),
+               "quadruped": (2587648, 1331200)}
+
+
+@pytest.mark.parametrize("name", list(SCENE_BYTES))
+def test_scene_bytes(name, steel):
+    """Packed rows take no more device memory: batches that filled it still fit, and a byte budget of
+    the serving loop admits as many instances."""
+    scene, opts = _sized(name)
+    pk = pack(scene, opts=opts, caps=auto_caps(scene))
+    for n, limit in zip((1, 200), SCENE_BYTES[name]):
+        g = Batch([pk] * n)
+        assert g.scene_bytes(n - 1) <= limit
+        g.close()
