@@ -7,7 +7,7 @@ import math
 import numpy as np
 import pytest
 
-from steel_webgpu_b200 import SceneBuilder, pack, synth
+from steel_webgpu_b200 import SceneBuilder, _lib, pack, synth
 from steel_webgpu_b200.sim import Batch, auto_caps
 
 pytestmark = pytest.mark.gpu
@@ -21,11 +21,13 @@ def _bits(a):
     return np.ascontiguousarray(a).view(np.uint32)
 
 
-def _same_as_oracle(pk, oracle_lib, frames, tiles=()):
+def _same_as_oracle(pk, oracle_lib, frames, tiles=(), team=0):
     o = oracle_lib.OracleSim(pk)
     g = Batch([pk])
     if tiles:
         g.set_tiles(*tiles)
+    if team:
+        g.set_team(team)
     for _ in range(2):
         o.step(frames)
         g.step(frames)
@@ -237,3 +239,38 @@ def test_scene_bytes(name, steel):
         g = Batch([pk] * n)
         assert g.scene_bytes(n - 1) <= limit
         g.close()
+
+
+def _heap(boxes):
+    """A plate that carries boxes: one body with more rows than a word of colors."""
+    b = SceneBuilder(fps=240, box_hulls="direct")
+    b.add_ground_plane(mu=0.6)
+    plate = b.add_body(xform=[0.0, 0.0, 0.051, 0, 0, 0, 1])
+    b.add_shape_box(plate, hx=0.7, hy=0.7, hz=0.05, mu=0.6)
+    for i in range(boxes):
+        body = b.add_body(xform=[0.25 * (i % 5) - 0.5, 0.25 * (i // 5) - 0.5, 0.203, 0, 0, 0, 1])
+        b.add_shape_box(body, hx=0.1, hy=0.1, hz=0.1, mu=0.6)
+    return b.finalize()
+
+
+def _overflow_rows(g):
+    """Rows of the first scene that have no color (of a table of 32), and all rows."""
+    start = g.read_words("sched", g.layout("S_CSTART"), 34, dtype=np.uint32).tolist()
+    return start[33] - start[32], start[33]
+
+
+@pytest.mark.parametrize("boxes", [8, 9, 25])
+@pytest.mark.parametrize("tiles,team", [((), 0), ((512, 4096), 0), ((32,), 0), ((), 2), ((), 5)])
+def test_packed_rows_without_a_color(boxes, tiles, team, steel, oracle_lib):
+    """The overflow color's rows, in global memory where the colors' are in shared memory (default
+    tiles), beside them in global memory (small budget) and in a team's."""
+    pk = pack(_heap(boxes), colorWords=1, caps=CAPS)
+    g = Batch([pk])
+    g.step(1)
+    g.sync()
+    over, rows = _overflow_rows(g)
+    assert 0 < over < rows
+    if not tiles and not team:  # the colors' rows fit what the solve has beside the bodies' twists
+        assert g.layout("solve_smem") > 64 * pk.NB + PACKED_TILE * (rows // 8 + 1)
+    g.close()
+    _same_as_oracle(pk, oracle_lib, 6, tiles, team)
