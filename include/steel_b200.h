@@ -231,7 +231,9 @@ int steel_trace_read(steel_batch* b, uint64_t* out, uint64_t words);
    shared-memory bulk copy before they record STEEL_E_TIMEOUT. steel_batch_create sets
    STEEL_WAIT_LIMIT_DEFAULT; 0 makes every staged scene's wait run out at once. After a timeout the
    kernel still waits, with the default limit, for its copy in flight, skips the scene and
-   returns, so the context stays usable. No counterpart in the reference (WebGPU has no bounded
+   returns, so the context stays usable. A quarter of it, 1 at least, bounds the passes of the row
+   coloring that waits without barriers; when they run out, the rows not yet colored go to the overflow
+   color and the same error is recorded. No counterpart in the reference (WebGPU has no bounded
    waits). */
 #define STEEL_WAIT_LIMIT_DEFAULT 16777216u
 int steel_debug_set_wait_limit(steel_batch* b, uint32_t rounds);

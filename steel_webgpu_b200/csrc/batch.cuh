@@ -32,8 +32,9 @@ struct BatchDev {
   uint32_t solve_ext;         // some scene has ANG_ART or CTI: launch the solve instances that carry them
   uint32_t solve_rows;        // ROWS_*: whether the scenes' contact rows are packed, launch the instance for that
   uint32_t block_threads;     // threads per prepare / solve block (one of BLOCK_SIZES)
-  uint32_t wait_limit;        // try_wait rounds of a shared-memory bulk copy (BULK_WAIT_LIMIT unless a test
-                              // lowers it to make the bounded wait run out)
+  uint32_t wait_limit;        // try_wait rounds of a shared-memory bulk copy, and four times the passes of a
+                              // thread over its bodies' row frontiers (BULK_WAIT_LIMIT unless a test lowers
+                              // it to make the bounded waits run out)
   unsigned long long* trace_prep;   // null, or [nscenes][3]: each scene's last k_prepare block, its start and
   unsigned long long* trace_solve;  // end (%globaltimer, ns) and SM; the same for k_solve (steel_trace)
   uint32_t team_blocks;       // nonzero: the batch's one scene is prepared and solved by this many
@@ -92,7 +93,6 @@ constexpr uint32_t RS_TILE = RS_THREADS * RS_ITEMS;
 constexpr uint32_t RS_DIGITS = 12;          // 96 key bits, 8 per digit
 constexpr uint32_t RS_SPIN_LIMIT = 1u << 22;  // polls of a preceding tile's status before giving up
 constexpr uint32_t TEAM_WAIT_LIMIT = 1u << 22;  // polls of a team launch's grid barrier before giving up
-constexpr uint32_t COLOR_WAIT_LIMIT = 1u << 22;  // passes of a thread over its bodies' frontiers before giving up
 // Team launches (team.cuh) on a batch of one scene: the default takes scenes of at least
 // TEAM_MIN_BODIES bodies or TEAM_MIN_ARTS articulations; such a scene's per-thread scratch has
 // slices for TEAM_SCRATCH_BLOCKS blocks, so the prepare's scratch passes spread over that many.

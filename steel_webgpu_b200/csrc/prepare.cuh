@@ -1256,7 +1256,7 @@ __device__ __forceinline__ void prepare_scene(const BatchDev& B, uint32_t sc, Te
                 if (o != 0xffffu) st_release_cta(&bpos[o], po + 1u);
               }
             }
-            if (left && ++passes >= COLOR_WAIT_LIMIT) {
+            if (left && ++passes >= max(B.wait_limit / 4u, 1u)) {
               atomicCAS(B.error, 0u, (uint32_t)ERR_COLOR_TIMEOUT);
               break;  // the rows left keep the overflow color
             }

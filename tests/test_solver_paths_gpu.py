@@ -274,3 +274,29 @@ def test_packed_rows_without_a_color(boxes, tiles, team, steel, oracle_lib):
         assert g.layout("solve_smem") > 64 * pk.NB + PACKED_TILE * (rows // 8 + 1)
     g.close()
     _same_as_oracle(pk, oracle_lib, 6, tiles, team)
+
+
+def test_coloring_wait_that_runs_out(steel, oracle_lib):
+    """One pass a thread is not enough for a body's rows: the step reports the timeout, with the rows left
+    in the overflow color; with the default limit back, a reset replays the scene bit for bit."""
+    pk = pack(_heap(8), colorWords=1, caps=CAPS)  # its lists fit shared memory: 12 rows a body
+    g = Batch([pk])
+    g.step(1)
+    g.sync()
+    colored = _overflow_rows(g)
+    g.reset()
+    _lib.check(_lib.load().steel_debug_set_wait_limit(g.h, 4))
+    g.step(1)
+    with pytest.raises(_lib.SteelError, match="coloring") as e:
+        g.sync()
+    assert e.value.code == 7
+    over, rows = _overflow_rows(g)
+    assert rows == colored[1] and over > colored[0]
+    assert np.isfinite(g.poses()).all()
+    _lib.check(_lib.load().steel_debug_set_wait_limit(g.h, 16777216))
+    g.reset()
+    o = oracle_lib.OracleSim(pk)
+    g.step(6)
+    o.step(6)
+    assert np.array_equal(_bits(o.read("poses")[:pk.NB * 8]), _bits(g.poses()))
+    g.close()
