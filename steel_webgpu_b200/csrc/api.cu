@@ -179,6 +179,22 @@ struct steel_batch {
 
 namespace {
 
+// Whether the records that build_levels follows lie in the packed arrays and name links of the scene.
+bool valid_links(const SceneHost& s) {
+  const SceneDev& d = s.d;
+  if (((uint64_t)d.SF_LINK + 6ull * d.NL) * 4u > s.statF.size()) return false;
+  if ((uint64_t)d.SU_ART + 4ull * d.NA > s.statU.size()) return false;
+  for (uint32_t l = 0; l < d.NL; l++) {
+    const float p = s.statF[4u * ((size_t)d.SF_LINK + l * 6u) + 1u];
+    if (!(p < (float)d.NL && p > -2147483648.0f)) return false;
+  }
+  for (uint32_t a = 0; a < d.NA; a++) {
+    const uint32_t* ai = s.statU.data() + d.SU_ART + a * 4u;
+    if ((uint64_t)ai[0] + ai[1] > d.NL) return false;
+  }
+  return true;
+}
+
 // The articulation trees by level (SceneDev::lt), from the packed link records.
 void build_levels(SceneHost& s) {
   SceneDev& d = s.d;
@@ -314,6 +330,7 @@ int build_scene(SceneHost& s, const steel_scene_desc& in, Layout& L, uint32_t th
   // Host copies: static data and initial state (the reference's reset() contents).
   s.statF.assign(in.statF, in.statF + in.statF_floats);
   s.statU.assign(in.statU, in.statU + in.statU_words);
+  if (!valid_links(s)) { why = "link records or articulation ranges out of range"; return STEEL_E_INVALID; }
   build_levels(s);
   s.pos0.resize(NB); s.rot0.resize(NB); s.lv0.resize(NB); s.av0.resize(NB);
   for (uint32_t b = 0; b < NB; b++) {

@@ -300,3 +300,19 @@ def test_coloring_wait_that_runs_out(steel, oracle_lib):
     o.step(6)
     assert np.array_equal(_bits(o.read("poses")[:pk.NB * 8]), _bits(g.poses()))
     g.close()
+
+
+@pytest.mark.parametrize("what", ["parent", "parent_nan", "range"])
+def test_links_out_of_range_are_refused(what, steel):
+    """The levels of the articulation trees are built on the host from the packed records: a parent or a
+    range of links that the scene does not have is an error there."""
+    pk = pack(_chains(3, 0.0), caps=CAPS)
+    if what == "range":
+        pk.statU = pk.statU.copy()
+        pk.statU[pk.C["SU_ART"] + 1] = pk.C["NL"] + 1
+    else:
+        pk.statF = pk.statF.copy()
+        pk.statF.reshape(-1, 4)[pk.C["SF_LINK"] + 6, 1] = np.nan if what == "parent_nan" else pk.C["NL"]
+    with pytest.raises(_lib.SteelError) as e:
+        Batch([pk])
+    assert e.value.code == 1
