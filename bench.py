@@ -206,7 +206,7 @@ def scene_counts(batch, pks):
 # (80,090 bodies, FP64 D-inverse, the 64-thread kernel instances and 12.9 KB staging budget the
 # autotuner picks for the bench batch; cold cache). Scaled by a batch's body count for the bench
 # line's roofline traffic; the narrow stage is k_narrow + k_narrow_jobs.
-NCU_TRAFFIC_PER_BODY = {"narrow": 2031.0, "prepare": 1902.0, "solve": 1575.0}
+NCU_TRAFFIC_PER_BODY = {"narrow": 2980.0, "prepare": 1682.0, "solve": 1510.0}
 
 
 def kernel_bytes(k: str, c: dict, rows_vec4: int, iterations: int) -> float:
@@ -215,8 +215,9 @@ def kernel_bytes(k: str, c: dict, rows_vec4: int, iterations: int) -> float:
     Terms follow the per-substep byte budget of the path: body static record 128 B and COM pose +
     twist 64 B read and written; shape record 112 B read, pose + AABB 64 B written; a pair 8 B
     written and read; a contact record 96 B written by narrow, read and written by the sort, read by
-    prepare; a row ROWS x 16 B written once and read every sweep with its 16 B impulse written; a
-    link block 1072 B read and written once, and per sweep 24 B twist read/written plus 432 B of
+    prepare; a row ROWS x 16 B written once and read once by the solve, which packs it (240 B written,
+    its impulse read back at the end) and reads 80 B of it every sweep (a visit that stops after the
+    normal impulse; others read it whole); a link block 1072 B read and written once, and per sweep 24 B twist read/written plus 432 B of
     motion subspace, U and D^-1 read.
     """
     NB, NS, NP, NC, NK, NL = c["NB"], c["NS"], c["pairs"], c["contacts"], c["rows"], c["NL"]
@@ -232,7 +233,7 @@ def kernel_bytes(k: str, c: dict, rows_vec4: int, iterations: int) -> float:
     if k == "prepare":
         return NB * (128 + 64) + NC * 96 + NK * rows_vec4 * 16 + NL * 2 * 1072
     if k == "solve":
-        return NK * rows_vec4 * 16 * (1 + I) + NK * 16 * (1 + I) + NB * (128 + 2 * 64) + NL * (2 * 1072 + I * (2 * 24 + 432))
+        return NK * (rows_vec4 * 16 + 240 + 16 + 80 * (1 + I)) + NB * (128 + 2 * 64) + NL * (2 * 1072 + I * (2 * 24 + 432))
     return 0.0
 
 

@@ -497,7 +497,9 @@ uint32_t stage_flags(const SceneDev& d, uint32_t budget, uint64_t body_cap, uint
 // STEEL_TEAM_AUTO takes scenes of at least TEAM_MIN_BODIES bodies or TEAM_MIN_ARTS articulations,
 // with eight threads per body or eight warps per articulation, capped by the blocks that fit the
 // GPU (a color's rows and the articulations spread over that many SMs: 128 quadrupeds and 8 chains
-// 7.7 ms a frame on 9 blocks, 6.1 on 72; an 8192-body pile 22.9 on 16, 21.5 on 128). Fewer
+// 5.11 ms a frame on 9 blocks, 4.11 on 36, 4.01 on 72, 3.96 on 148; an 8192-body pour 25.5 on 8, 24.0 on
+// 16, 22.9 on 128; TEAM_MIN_BODIES is where teams were first tried, a 1500-body pour would gain too, 9.8
+// on one block, 8.2 on 16). Fewer
 // than two blocks: the one-block path. `strict`: a request for more blocks than fit, or under
 // smaller tiles, is an error (steel_set_team) rather than capped (a later change of tiles).
 int team_blocks_for(const steel_batch* b, uint32_t req, bool strict, uint32_t* out) {
@@ -737,7 +739,11 @@ int apply_tiles(steel_batch* b, const steel_tiles& t) {
 // Block size a batch starts with: 512 for no more scenes than SMs. For more, the largest of 32, 64 and
 // 128 that keeps all of them resident at once (a second wave of blocks costs as much as the first:
 // 1024 quadrupeds 5.9 ms a frame on 128 threads, 4.6 on 64; 1500 arms 1.35 and, on 32, 0.68), but 64
-// at least for scenes of more than 32 bodies on average, whose parallel passes need the threads.
+// at least for scenes of more than 32 bodies on average, the size from which the uneven batches (142 on
+// average) were found to want the threads. On 32, 64 and 128 threads, ms a frame: 400 scenes of 20
+// stacked boxes 7.8, 7.3, 6.9 (takes 128); 1000 of 48 42.2, 39.2, 44.1 (64); 2000 of 20 23.2, 25.9, 30.4
+// and of a 30-link chain 6.4, 7.4, 9.7 (32); just above the line 64 costs more: 2000 of 33 boxes 52.7,
+// 58.6, 66.1 and of three quadrupeds 11.5, 12.5, 15.3.
 uint32_t default_threads(const steel_batch* b) {
   if (b->max_threads == (uint32_t)BIG_THREADS) return b->max_threads;
   const uint64_t n = b->sc.size();

@@ -118,10 +118,14 @@ struct RadixDev {
 // Shared-memory staging of a scene inside k_prepare / k_solve. A scene is staged when its part
 // fits the cap; the launch's dynamic shared memory is the largest staged scene's need.
 enum : uint32_t { STAGE_LINKS = 1u, STAGE_BODIES = 2u, STAGE_QD = 4u, STAGE_WMASK = 8u };
-// Caps keep four prepare / solve blocks resident per SM.
+// Caps on what a block stages of each part; larger parts stay in global memory and are read through L1.
+// Twists and impulses may take a third of what the batch's resident blocks leave a block, where that is
+// more than their cap (apply_tiles).
 constexpr uint32_t STAGE_LINK_CAP = 44u * 1024u;   // link blocks (NL * 1072 B), batches of no more scenes than SMs
-constexpr uint32_t STAGE_LINK_CAP_MANY = 16u * 1024u;  // larger batches: a quadruped's, not a 40-link chain's (43 KB, which
-                                                       // serve better as L1: served instances 5.2 -> 4.2 ms a frame)
+// The same in larger batches, where several blocks share an SM: beyond 15 links the memory serves better
+// as L1. Chains of 16, 20, 28 and 40 links, 200 scenes: 1.03, 1.28, 1.78 and 2.74 ms a frame, staged
+// 1.05, 1.32, 1.97 and 3.02; 320 served instances 5.2 -> 4.6 ms a frame.
+constexpr uint32_t STAGE_LINK_CAP_MANY = 16u * 1024u;
 constexpr uint32_t STAGE_BODY_CAP = 8u * 1024u;    // twists + impulses (NB * 64 B)
 constexpr uint32_t STAGE_QD_CAP = 8u * 1024u;      // generalized velocities of the solve (ND * 4 B)
 constexpr uint32_t STAGE_WMASK_CAP = 16u * 1024u;  // per-body color masks (NB * NCOLW words)

@@ -1169,7 +1169,7 @@ __device__ __forceinline__ void prepare_scene(const BatchDev& B, uint32_t sc, Te
         // its lower body, which then moves both frontiers on. The threads go over their bodies without
         // barriers: a body's masks are written before its frontier moves (release) and read after
         // it is seen to have (acquire), and the lowest uncolored row is always ready, so every pass of
-        // its thread colors it. On 64 boxes this took the prepare from 166 to 140 us. It needs the
+        // its thread colors it. On 64 boxes this took the prepare from 166 to 126 us. It needs the
         // lists in shared memory, beyond the scene's staging (from global memory the acquiring loads
         // made an 8192-body pile's prepare 2.44 ms against 1.64 ms); other scenes take the rounds
         // below.
